@@ -4,8 +4,8 @@
 // run-loop control). The phases of an attempt are separated by grid-wide
 // barriers (cooperative groups; the cooperative launch guarantees that every
 // block is resident, and every block takes every barrier):
-//   zero the reduction slots and limiter counters | stage 1 | limiter scan |
-//   limiter rewrite | stage 2 | ... | stage 3 | ... | report + control
+//   zero the reduction slots | stage 1 | limiter | stage 2 | limiter |
+//   stage 3 | limiter | report + control
 // Finished instances are skipped by the bodies; the loop ends early once no
 // instance is active. The per-tile and per-element work is exactly the
 // stage / limiter / control code of the separate launches, so the results are
@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(2 * BatchShape<R>::EPB, BatchShape<R>::MINB)
     batch_persistent_kernel(const BatchParams B) {
   using SH = BatchShape<R>;
   constexpr int EPB = SH::EPB, BS = 2 * EPB;
+  static_assert(BS == LIMIT_BS, "the limiter runs in the stage tile's block");
   constexpr int MODE = PHI == LIM_UNLIMITED ? MODE_UNLIMITED : MODE_LIMITED;
   namespace cgr = cooperative_groups;
   cgr::grid_group grid = cgr::this_grid();
@@ -73,11 +74,9 @@ __global__ void __launch_bounds__(2 * BatchShape<R>::EPB, BatchShape<R>::MINB)
   lp.avg = s.averages;
   lp.aux = s.element_aux;
   lp.acc = s.acc;
-  lp.list = s.limit_list + LIMIT_LIST_HEADER;
 
   for (int it = 0; it < B.attempts; ++it) {
     for (int i = gtid; i < 3 * n; i += gthreads) reset_acc_one(s.acc, i);
-    if (gtid < 4) s.limit_list[gtid] = 0;
     grid.sync();
     for (int k = 1; k <= 3; ++k) {
       p.stage_idx = k;
@@ -88,10 +87,10 @@ __global__ void __launch_bounds__(2 * BatchShape<R>::EPB, BatchShape<R>::MINB)
       grid.sync();
       if constexpr (PHI != LIM_UNLIMITED) {
         lp.stage_idx = k;
-        lp.count = s.limit_list + k;
-        for (int e0 = blockIdx.x * BS; e0 < K; e0 += gridDim.x * BS) limit_scan_body<R, PHI, BS>(lp, e0);
-        grid.sync();
-        limit_rewrite_body<R, PHI>(lp);
+        for (int e0 = blockIdx.x * LIMIT_BS; e0 < K; e0 += gridDim.x * LIMIT_BS) {
+          limit_block_body<R, PHI, LIMIT_BS, LIMIT_BS>(lp, e0);
+          __syncthreads();  // the next block of elements reuses the shared list
+        }
         grid.sync();
       }
     }

@@ -32,9 +32,6 @@ constexpr double POSITIVITY_FLOOR = 1e-13;    // limiting.py:28
 constexpr int BISECTION_STEPS = 60;           // limiting.py:29
 
 enum { MODE_RHS = 0, MODE_LIMITED = 1, MODE_UNLIMITED = 2 };
-// CfdSolver.limit_list: [LIMIT_LIST_HEADER] counters (index = RK stage, 0 for
-// cfd_limit), then the element list
-constexpr int LIMIT_LIST_HEADER = CFD_LIMIT_LIST_HEADER;
 // bits 0-1 decide admissibility; bit 2 marks a NaN CFL step (time_step -> NaN)
 enum { FLAG_NONFINITE = 1, FLAG_BAD_AVERAGE = 2, FLAG_NAN_DT = 4, FLAG_ADMISSIBILITY = 3 };
 
@@ -89,6 +86,15 @@ struct Red {
     tr = 0;
     fl = 0;
   }
+  __device__ void merge(const Red& r) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) b[c] += r.b[c];
+    kr = min(kr, r.kr);
+    kp = min(kp, r.kp);
+    kd = min(kd, r.kd);
+    tr += r.tr;
+    fl |= r.fl;
+  }
 };
 
 // Appends e to list[] where flag is set, with one atomic per warp on the
@@ -108,11 +114,50 @@ __device__ __forceinline__ void commit_one(const Red& r, CfdStageAcc* a) {
 #pragma unroll
   for (int c = 0; c < 4; ++c)
     if (r.b[c] != 0.0) atomicAdd(&a->boundary_flux[c], r.b[c]);
-  if (r.kr != KEY_EMPTY) atomicMin(&a->min_rho_key, r.kr);
-  if (r.kp != KEY_EMPTY) atomicMin(&a->min_p_key, r.kp);
-  if (r.kd != KEY_EMPTY) atomicMin(&a->dt_key, r.kd);
+  // The minima only fall, so a value that is not below the one read here (even
+  // a stale one) cannot lower it: the atomic is left out. Every block of the
+  // mesh commits to the same three words, where atomics serialise.
+  const volatile CfdStageAcc* seen = a;
+  const unsigned long long kr = seen->min_rho_key, kp = seen->min_p_key, kd = seen->dt_key;
+  if (r.kr < kr) atomicMin(&a->min_rho_key, r.kr);
+  if (r.kp < kp) atomicMin(&a->min_p_key, r.kp);
+  if (r.kd < kd) atomicMin(&a->dt_key, r.kd);
   if (r.tr) atomicAdd(&a->troubled, r.tr);
   if (r.fl) atomicOr(&a->flags, r.fl);
+}
+
+// Least key of the warp: the high words, then the low words of the lanes that
+// hold the least high word (two 32-bit warp reductions).
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+  const unsigned hi = (unsigned)(k >> 32), h = __reduce_min_sync(0xffffffffu, hi);
+  const unsigned l = __reduce_min_sync(0xffffffffu, hi == h ? (unsigned)k : 0xffffffffu);
+  return ((unsigned long long)h << 32) | l;
+}
+
+// Block reduction and commit of the minima, the troubled count and the flags
+// (no boundary flux) to one stage accumulator. All threads of the block call it.
+__device__ __forceinline__ void commit_keys(const Red& r, CfdStageAcc* acc) {
+  __shared__ unsigned long long s_key[3];
+  __shared__ int s_sum[2];
+  if (threadIdx.x < 3) s_key[threadIdx.x] = KEY_EMPTY;
+  if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
+  const unsigned long long kr = warp_min_key(r.kr), kp = warp_min_key(r.kp), kd = warp_min_key(r.kd);
+  const int tr = __reduce_add_sync(0xffffffffu, r.tr), fl = __reduce_or_sync(0xffffffffu, (unsigned)r.fl);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(&s_key[0], kr);
+    atomicMin(&s_key[1], kp);
+    atomicMin(&s_key[2], kd);
+    if (tr) atomicAdd(&s_sum[0], tr);
+    if (fl) atomicOr(&s_sum[1], fl);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    Red t;
+    t.init();
+    t.kr = s_key[0], t.kp = s_key[1], t.kd = s_key[2], t.tr = s_sum[0], t.fl = s_sum[1];
+    commit_one(t, acc);
+  }
 }
 
 // Reduce over the block and commit with one set of atomics when every live
@@ -257,72 +302,74 @@ __device__ __forceinline__ void cell_average(const R (&q)[NP][4], double a[4]) {
   }
 }
 
-// Zhang-Shu positivity scaling of one element toward its average, in double
-// and in the reference's operation order (limiting.py:166-200). q is the
-// element's nodal state in registers. Returns true if q changed.
-template <typename R>
-__device__ __forceinline__ bool positivity(R (&q)[NP][4], const double a[4], double gm1, double* theta_out = nullptr,
-                                           int* node_out = nullptr) {
-  const double pa = pressure_x(a[0], a[1], a[2], a[3], gm1);
-  const double eps = jmin(POSITIVITY_FLOOR, jmin(a[0], pa));
-  const double pt = pressure_target<R>(eps, pa, a[3], gm1);
-  double rmin = (double)q[0][0];
-#pragma unroll
-  for (int i = 1; i < NP; ++i) rmin = jmin(rmin, (double)q[i][0]);
-  bool changed = false;
-  if (rmin < eps) {
-    const double span = xsub(a[0], rmin);
-    const double theta = jmin(jmax(xdiv(xsub(a[0], eps), span), 0.0), 1.0);
-#pragma unroll
-    for (int i = 0; i < NP; ++i)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) q[i][c] = (R)xadd(a[c], xmul(theta, xsub((double)q[i][c], a[c])));
-    changed = true;
-  }
-  unsigned need = 0;
-#pragma unroll
-  for (int i = 0; i < NP; ++i)
-    if (pressure_near(q[i][0], q[i][1], q[i][2], q[i][3], gm1, pt) < pt) need |= 1u << i;
-  if (theta_out) {
-    *theta_out = 1.0;
-    *node_out = -1;
-  }
-  if (!need) return changed;
-  double theta = 1.0;
+// Root of the pressure scaling by bisection (limiting.py:183-200): the lower
+// end after BISECTION_STEPS halvings of [0, 1] on pressure(a + theta d) >= pt,
+// bit for bit, without evaluating the halvings whose outcome is certain.
+//
+// With positive density at both ends the pressure is concave along the
+// segment, so if it exceeds pt by more than the evaluation's rounding at 0 and
+// at lo_k, it does so on all of [0, lo_k]; and if it lies below pt by more
+// than that at hi_k, it does so on all of [hi_k, 1]. The first k halvings then
+// all have the outcome that leads to [lo_k, hi_k], a dyadic interval around
+// the root of the quadratic rho (E - pt / (gamma - 1)) - |m|^2 / 2 (every
+// midpoint down to 2^-48 is exact). `delta` bounds the rounding of p at any
+// point of the segment: the points' own rounding and some ten operations, each
+// relative 2^-53, through the pressure's sensitivity to rho, m and E, with the
+// velocities bounded by their end values (they are monotone along the
+// segment): 5 units, taken twice (the check's own value and the certain one)
+// and rounded up to 16. Where a check fails the interval is widened, and in the
+// end the loop runs from [0, 1] as written. The remaining halvings go two at a
+// time, their three candidate points evaluated together (the loop is one
+// serial chain of divisions, 125 cycles each), and end once lo and hi are
+// neighbours: the midpoint then rounds to one of them, both known.
+__device__ __forceinline__ double pressure_theta(const double a[4], double d0, double d1, double d2, double d3,
+                                                 double gm1, double pt) {
+  auto at = [&](double th) {
+    return pressure_x(xadd(a[0], xmul(th, d0)), xadd(a[1], xmul(th, d1)), xadd(a[2], xmul(th, d2)),
+                      xadd(a[3], xmul(th, d3)), gm1);
+  };
+  double lo = 0.0, hi = 1.0;
+  int it = 0;
+  const double e0 = a[0] + d0;
+  if (a[0] > 0.0 && e0 > 0.0) {
+    const double t = a[3] - pt / gm1;
+    const double qa = d0 * d3 - 0.5 * (d1 * d1 + d2 * d2), qb = a[0] * d3 + d0 * t - (a[1] * d1 + a[2] * d2);
+    const double qc = a[0] * t - 0.5 * (a[1] * a[1] + a[2] * a[2]);
+    const double s = sqrt(qb * qb - 4.0 * qa * qc);
+    const double root = qb < 0.0 ? 2.0 * qc / (s - qb) : -0.5 * (qb + s) / qa;
+    const double ia = 1.0 / a[0], ie = 1.0 / e0;
+    const double u = fmax(fabs(a[1] * ia), fabs((a[1] + d1) * ie)), v = fmax(fabs(a[2] * ia), fabs((a[2] + d2) * ie));
+    const double delta = 16.0 * 1.1102230246251565e-16 * gm1 *
+                         (fabs(a[3]) + fabs(d3) + u * (fabs(a[1]) + fabs(d1)) + v * (fabs(a[2]) + fabs(d2)) +
+                          (u * u + v * v) * (fabs(a[0]) + fabs(d0)));
+    // 2^-k about 8 delta / |dp/dtheta| at the root, where |d(quadratic)/dtheta| = s
+    const double w = 8.0 * delta * (a[0] + root * d0) / (gm1 * s);
+    if (root >= 0.0 && root < 1.0 && w > 0.0 && w < 0.0625 && at(0.0) - pt > delta) {
+      int k = min(48, -1 - ilogb(w)) & ~1;
 #pragma unroll 1
-  for (int i = 0; i < NP; ++i) {
-    if (!((need >> i) & 1u)) continue;
-    double qi[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      // select node i without dynamic register indexing
-      double v = 0.0;
-#pragma unroll
-      for (int j = 0; j < NP; ++j) v = (j == i) ? (double)q[j][c] : v;
-      qi[c] = v;
+      for (; k >= 4; k -= 4) {
+        const double n = ldexp(1.0, k), h = ldexp(1.0, -k);
+        const double l = floor(root * n) * h, r = l + h;
+        if (r <= 1.0 && (l == 0.0 || at(l) - pt > delta) && pt - at(r) > delta) {
+          lo = l;
+          hi = r;
+          it = k;
+          break;
+        }
+      }
     }
-    const double d0 = xsub(qi[0], a[0]), d1 = xsub(qi[1], a[1]), d2 = xsub(qi[2], a[2]), d3 = xsub(qi[3], a[3]);
-    double lo = 0.0, hi = 1.0;
+  }
 #pragma unroll 1
-    for (int it = 0; it < BISECTION_STEPS; ++it) {
-      const double mid = xmul(0.5, xadd(lo, hi));
-      const bool ok = pressure_x(xadd(a[0], xmul(mid, d0)), xadd(a[1], xmul(mid, d1)), xadd(a[2], xmul(mid, d2)),
-                                 xadd(a[3], xmul(mid, d3)), gm1) >= pt;
-      lo = ok ? mid : lo;
-      hi = ok ? hi : mid;
-    }
-    if (theta_out && lo < theta) *node_out = i;
-    theta = jmin(theta, lo);
+  for (; it < BISECTION_STEPS; it += 2) {
+    const double mid = xmul(0.5, xadd(lo, hi));
+    if ((mid == lo || mid == hi) && lo > 0.0 && hi < 1.0) break;
+    const double ml = xmul(0.5, xadd(lo, mid)), mr = xmul(0.5, xadd(mid, hi));
+    const bool ok = at(mid) >= pt, okl = at(ml) >= pt, okr = at(mr) >= pt;
+    const double l = ok ? (okr ? mr : mid) : (okl ? ml : lo);
+    hi = ok ? (okr ? hi : mr) : (okl ? mid : ml);
+    lo = l;
   }
-  if (theta_out) *theta_out = theta;
-  if (theta < 1.0) {
-#pragma unroll
-    for (int i = 0; i < NP; ++i)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) q[i][c] = (R)xadd(a[c], xmul(theta, xsub((double)q[i][c], a[c])));
-    changed = true;
-  }
-  return changed;
+  return lo;
 }
 
 // Nodal minima (density, pressure; NaN ignored), max wave speed and finiteness.

@@ -92,9 +92,8 @@ __global__ void __launch_bounds__(BS) dt_kernel(CfdMesh m, const R* __restrict__
   block_commit<BS>(red, live, inst, acc, 3, 2);
 }
 
-__global__ void reset_acc_kernel(CfdStageAcc* acc, int n, int* list_counters) {
+__global__ void reset_acc_kernel(CfdStageAcc* acc, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 4 && list_counters) list_counters[i] = 0;  // the two-pass limiter's per-stage counters
   if (i < n) reset_acc_one(acc, i);
 }
 
@@ -318,56 +317,25 @@ static void launch_stage(const CfdSolver* s, const StageParams& p, int mode, cud
   }
 }
 template <typename R, int PHI>
-static void launch_limit_bs(const LimitParams& p, int bs, cudaStream_t st) {
-  const unsigned g = blocks_for(p.m.num_elements, bs);
-  if (bs == 64) limit_kernel<R, PHI, 64><<<g, 64, 0, st>>>(p);
-  else if (bs == 256) limit_kernel<R, PHI, 256><<<g, 256, 0, st>>>(p);
-  else limit_kernel<R, PHI, 128><<<g, 128, 0, st>>>(p);
+static void launch_limit_phi(const LimitParams& p, cudaStream_t st) {
+  const int n = p.m.num_elements;
+  if (n <= LIMIT_DIRECT_MAX) limit_kernel<R, PHI, LIMIT_BS / HALF><<<blocks_for(n, LIMIT_BS / HALF), LIMIT_BS, 0, st>>>(p);
+  else if (n <= LIMIT_SCAN32_MAX) limit_kernel<R, PHI, 32><<<blocks_for(n, 32), LIMIT_BS, 0, st>>>(p);
+  else limit_kernel<R, PHI, LIMIT_BS><<<blocks_for(n, LIMIT_BS), LIMIT_BS, 0, st>>>(p);
 }
 template <typename R>
-static void launch_limit_phi(const LimitParams& p, int lim, int bs, cudaStream_t st) {
+static void launch_limit_lim(const LimitParams& p, int lim, cudaStream_t st) {
   switch (lim) {
-    case 0: launch_limit_bs<R, 0>(p, bs, st); break;
-    case 1: launch_limit_bs<R, 1>(p, bs, st); break;
-    case 2: launch_limit_bs<R, 2>(p, bs, st); break;
-    case 3: launch_limit_bs<R, 3>(p, bs, st); break;
-    default: launch_limit_bs<R, 4>(p, bs, st); break;
+    case 0: launch_limit_phi<R, 0>(p, st); break;
+    case 1: launch_limit_phi<R, 1>(p, st); break;
+    case 2: launch_limit_phi<R, 2>(p, st); break;
+    case 3: launch_limit_phi<R, 3>(p, st); break;
+    default: launch_limit_phi<R, 4>(p, st); break;
   }
 }
-template <typename R, int PHI>
-static void launch_limit_two_pass(const LimitParams& p, int bs, cudaStream_t st) {
-  const unsigned g = blocks_for(p.m.num_elements, bs);
-  if (bs == 64) limit_scan_kernel<R, PHI, 64><<<g, 64, 0, st>>>(p);
-  else if (bs == 256) limit_scan_kernel<R, PHI, 256><<<g, 256, 0, st>>>(p);
-  else limit_scan_kernel<R, PHI, 128><<<g, 128, 0, st>>>(p);
-  // the list's length is only known on the device: four threads per listed
-  // element, enough for a sixteenth of the elements in one sweep (blocks
-  // beyond the list end exit at once; a longer list is swept grid-stride)
-  const unsigned full = blocks_for(p.m.num_elements, 64), cap = 32 * 148;
-  limit_rewrite_kernel<R, PHI><<<full < cap ? full : cap, 64, 0, st>>>(p);
-}
-template <typename R>
-static void launch_limit_two_pass_phi(const LimitParams& p, int lim, int bs, cudaStream_t st) {
-  switch (lim) {
-    case 0: launch_limit_two_pass<R, 0>(p, bs, st); break;
-    case 1: launch_limit_two_pass<R, 1>(p, bs, st); break;
-    case 2: launch_limit_two_pass<R, 2>(p, bs, st); break;
-    case 3: launch_limit_two_pass<R, 3>(p, bs, st); break;
-    default: launch_limit_two_pass<R, 4>(p, bs, st); break;
-  }
-}
-// With a limit_list scratch the limiter runs in two passes (scan + rewrite
-// of the listed elements); without one, in one pass.
-static void launch_limit(const CfdSolver* s, LimitParams p, cudaStream_t st) {
-  if (s->limit_list) {
-    p.count = s->limit_list + (p.stage_idx >= 0 && p.stage_idx <= 3 ? p.stage_idx : 0);
-    p.list = s->limit_list + LIMIT_LIST_HEADER;
-    if (s->precision == CFD_FP64) launch_limit_two_pass_phi<double>(p, s->limiter, bs_of(s), st);
-    else launch_limit_two_pass_phi<float>(p, s->limiter, bs_of(s), st);
-    return;
-  }
-  if (s->precision == CFD_FP64) launch_limit_phi<double>(p, s->limiter, bs_of(s), st);
-  else launch_limit_phi<float>(p, s->limiter, bs_of(s), st);
+static void launch_limit(const CfdSolver* s, const LimitParams& p, cudaStream_t st) {
+  if (s->precision == CFD_FP64) launch_limit_lim<double>(p, s->limiter, st);
+  else launch_limit_lim<float>(p, s->limiter, st);
 }
 template <typename R>
 static void launch_dt(const CfdSolver* s, const void* q, cudaStream_t st) {
@@ -376,7 +344,7 @@ static void launch_dt(const CfdSolver* s, const void* q, cudaStream_t st) {
 }
 static void reset_acc(const CfdSolver* s, cudaStream_t st) {
   const int n = 3 * s->mesh.num_instances;
-  reset_acc_kernel<<<blocks_for(n > 4 ? n : 4, 128), 128, 0, st>>>(s->acc, n, s->limit_list);
+  reset_acc_kernel<<<blocks_for(n, 128), 128, 0, st>>>(s->acc, n);
 }
 
 extern "C" {
@@ -443,8 +411,6 @@ int cfd_limit(const CfdSolver* s, const void* q_in, void* q_out, int32_t* troubl
   if (!q_in || !q_out || !troubled || !s->averages || !s->element_aux) return fail(CFD_E_ARG, "cfd_limit: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   if (cudaMemsetAsync(troubled, 0, sizeof(int32_t) * s->mesh.num_instances, st) != cudaSuccess)
-    return check_launch("cfd_limit: memset");
-  if (s->limit_list && cudaMemsetAsync(s->limit_list, 0, sizeof(int32_t), st) != cudaSuccess)
     return check_launch("cfd_limit: memset");
   const int bs = 128;
   const unsigned g = blocks_for(s->mesh.num_elements, bs);

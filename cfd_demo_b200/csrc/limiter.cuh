@@ -1,6 +1,6 @@
 // limiter.cuh — the Cockburn-Shu troubled-cell limiter and the Zhang-Shu
 // positivity limiter of a stage state (limiting.py:136-216 of CFD-demo), as
-// per-element bodies and the one-pass / two-pass kernels that run them.
+// per-element bodies and the kernel that runs them.
 // Included by common.cuh inside namespace cfd.
 #pragma once
 
@@ -19,397 +19,64 @@ struct LimitParams {
   CfdStageAcc* acc;       // stage mode
   int32_t* troubled_out;  // cfd_limit mode
   double* pos_out;        // optional [2][ld]: pressure-scaling theta and its critical node
-  int* list;              // two-pass form: elements for the rewrite pass, and
-  int* count;             // their number (zeroed before the scan)
   uint8_t* flags;         // optional [ld]: troubled-cell indicator per element
 };
 
-// Troubled-cell detection of element e (limiting.py:128-151): the scaled
-// neighbour differences (Cockburn-Shu coefficients, neighbour or ghost
-// averages) and whether a density or energy trace at a face midpoint leaves
-// its minmod bound. q is the stage state (element-major rows).
-template <typename R, int PHI>
-__device__ __forceinline__ bool limit_detect(const LimitParams& P, int e, const R* __restrict__ q, const double a[4],
-                                             int finfo, double det_tol, R (&scaled)[3][4]) {
-  const CfdMesh& m = P.m;
-  const int ld = m.ld;
-  bool troubled = false;
-  {
-      // neighbour / ghost averages (limiting.py:128-133), unfused as in NumPy
-      R diff[3][4];
-      const double* fgd = m.face_geo;
-#pragma unroll
-      for (int f = 0; f < 3; ++f) {
-        const int kind = (finfo >> (8 * f)) & 3;
-        double na[4];
-        if (kind == CFD_FACE_INTERIOR) {
-          const int nb = m.neighbor[f * ld + e];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) na[c] = P.avg[c * ld + nb];
-        } else if (kind == CFD_FACE_SLIP_WALL) {
-          const double nx = fgd[(3 * f) * ld + e], ny = fgd[(3 * f + 1) * ld + e];
-          const double mn = xadd(xmul(a[1], nx), xmul(a[2], ny));
-          na[0] = a[0];
-          na[1] = xsub(a[1], xmul(xmul(2.0, mn), nx));
-          na[2] = xsub(a[2], xmul(xmul(2.0, mn), ny));
-          na[3] = a[3];
-        } else {
-          // the ghost average: the fixed state, or the exact state's row after its node rows
-          const int row = m.neighbor[f * ld + e] + (kind == CFD_FACE_EXACT_STATE ? NFP : 0);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) na[c] = m.bc_states[row * 4 + c];
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) diff[f][c] = (R)xsub(na[c], a[c]);
-      }
-      const R* __restrict__ cs = GeoPtr<R>::cs(m);
-#pragma unroll
-      for (int f = 0; f < 3; ++f) {
-        const int pf = (finfo >> (8 * f + 4)) & 3;
-        const R al = cs[f * ld + e], be = cs[(3 + f) * ld + e];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const R pd = pf == 0 ? diff[0][c] : (pf == 1 ? diff[1][c] : diff[2][c]);
-          scaled[f][c] = xmul((R)NEIGHBOR_FACTOR, xadd(xmul(al, diff[f][c]), xmul(be, pd)));
-        }
-      }
-      // detection on rho and E at the three face midpoints (limiting.py:147-151)
-#pragma unroll
-      for (int f = 0; f < 3; ++f) {
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-          const int c = cc == 0 ? 0 : 3;
-          const R tr = xsub(q[(c * NP + tab::MID_NODES[f]) * ld + e], (R)a[c]);
-          const R ex = abs_(xsub(minmod2(tr, scaled[f][c]), tr));
-          troubled |= (double)ex > xmul(det_tol, fabs(a[c]));
-        }
-      }
-      }
-  return troubled;
+// The stage state the limiter works on, in place.
+template <typename R>
+__device__ __forceinline__ R* limit_state(const LimitParams& P, int par) {
+  return P.stage_idx == 0 ? (R*)P.q_io : P.stage_idx == 2 ? (R*)P.stage : (R*)(par ? P.x0 : P.x1);
 }
 
-// Cockburn-Shu troubled-cell limiter (limiting.py:136-163) followed by the
-// positivity limiter (limiting.py:166-200), in place on the stage state, for
-// element e of instance inst. PART 0: everything in one pass; PART 1 (scan):
-// elements the limiters leave as they are contribute their minima, the others
-// are only marked `listed`; PART 2: the rewrite of a listed element.
-template <typename R, int PHI, int PART>
-__device__ __forceinline__ void limit_body(const LimitParams& P, int e, int par, Red& red, bool& listed) {
-  const CfdMesh& m = P.m;
-  const int ld = m.ld;
-  {
-    R* __restrict__ q;
-    if (P.stage_idx == 0) {
-      q = (R*)P.q_io;
-    } else if (P.stage_idx == 2) {
-      q = (R*)P.stage;
-    } else {
-      q = (R*)(par ? P.x0 : P.x1);
-    }
-    const double gm1 = P.gamma - 1.0;
-    double a[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) a[c] = P.avg[c * ld + e];
-    const double pa = pressure_x(a[0], a[1], a[2], a[3], gm1);
-    const double eps = jmin(POSITIVITY_FLOOR, jmin(a[0], pa));
-    const double pt = pressure_target<R>(eps, pa, a[3], gm1);
-    const double det_tol = sizeof(R) == 8 ? DETECTION_TOLERANCE : DETECTION_TOLERANCE_FP32;
-    const int finfo = m.face_info[e];
-    bool troubled = false;
-    R scaled[3][4];
-    if (PHI != LIM_UNLIMITED) troubled = limit_detect<R, PHI>(P, e, q, a, finfo, det_tol, scaled);
-    if (PART != 2 && P.flags) P.flags[e] = troubled ? 1 : 0;
-    const double rmin0 = P.aux[e], pmin0 = P.aux[ld + e];
-    const bool need_pos = (rmin0 < eps) || (pmin0 < pt);
-    if (!troubled && !need_pos) {
-      red.kr = dkey(rmin0);
-      red.kp = dkey(pmin0);
-      if (P.stage_idx == 3) {
-        const double d = m.dt_geo[e] / P.aux[2 * ld + e];
-        red.kd = dkey(d);
-        if (d != d) red.fl |= FLAG_NAN_DT;
-      }
-    } else {
-      if (PART == 1) {  // the scan pass lists the element for the rewrite pass
-        listed = true;
-        return;
-      }
-      R s[NP][4];
-#pragma unroll
-      for (int i = 0; i < NP; ++i)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) s[i][c] = q[(c * NP + i) * ld + e];
-      if (troubled) {
-        // P1 midpoint values, phi-limited deltas, +/- rescaling, linear rebuild
-        // (limiting.py:153-162), in NumPy's operation order
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const R ac = (R)a[c];
-          R deltas[3];
-          R pos = R(0), neg = R(0);
-#pragma unroll
-          for (int f = 0; f < 3; ++f) {
-            R pr = xmul((R)tab::P1MID[f][0], s[0][c]);
-#pragma unroll
-            for (int i = 1; i < NP; ++i) pr = xadd(pr, xmul((R)tab::P1MID[f][i], s[i][c]));
-            pr = xsub(pr, ac);
-            R d = R(0);
-            if (pr != R(0)) d = xmul(pr, jmin(R(1), phi<R, PHI>(xdiv(scaled[f][c], pr))));
-            deltas[f] = d;
-            pos = f == 0 ? jmax(d, R(0)) : xadd(pos, jmax(d, R(0)));
-            neg = f == 0 ? jmax(-d, R(0)) : xadd(neg, jmax(-d, R(0)));
-          }
-          const R thp = pos > R(0) ? jmin(R(1), xdiv(neg, pos)) : R(0);
-          const R thn = neg > R(0) ? jmin(R(1), xdiv(pos, neg)) : R(0);
-#pragma unroll
-          for (int f = 0; f < 3; ++f)
-            deltas[f] = xsub(xmul(thp, jmax(deltas[f], R(0))), xmul(thn, jmax(-deltas[f], R(0))));
-#pragma unroll
-          for (int i = 0; i < NP; ++i) {
-            R v = xmul((R)tab::LINBASIS[i][0], deltas[0]);
-            v = xadd(v, xmul((R)tab::LINBASIS[i][1], deltas[1]));
-            v = xadd(v, xmul((R)tab::LINBASIS[i][2], deltas[2]));
-            s[i][c] = xadd(ac, v);
-          }
-        }
-        red.tr = 1;
-      }
-      if (P.pos_out) {
-        double th;
-        int node;
-        positivity<R>(s, a, gm1, &th, &node);
-        P.pos_out[e] = th;
-        P.pos_out[ld + e] = (double)node;
-      } else {
-        positivity<R>(s, a, gm1);
-      }
-#pragma unroll
-      for (int i = 0; i < NP; ++i)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) q[(c * NP + i) * ld + e] = s[i][c];
-      double rmin, pmin, lam;
-      bool finite;
-      element_stats<R>(s, gm1, P.gamma, rmin, pmin, lam, finite);
-      if (!finite) red.fl |= FLAG_NONFINITE;
-      red.kr = dkey(rmin);
-      red.kp = dkey(pmin);
-      if (P.stage_idx == 3) {
-        const double d = m.dt_geo[e] / lam;
-        red.kd = dkey(d);
-        if (d != d) red.fl |= FLAG_NAN_DT;
-      }
-    }
-    }
-}
-
-template <typename R, int PHI, int BS>
-__global__ void __launch_bounds__(BS) limit_kernel(const LimitParams P) {
-  const CfdMesh& m = P.m;
-  const int e = blockIdx.x * BS + threadIdx.x;
-  bool live = e < m.num_elements;
-  int inst = 0;
-  if (live && m.instance) inst = m.instance[e];
-  if (inst < 0) {  // padding between instances
-    live = false;
-    inst = 0;
-  }
-  int par = 0;
-  if (live && P.ctl) {
-    live = P.ctl[inst].status == CFD_RUN_ACTIVE;
-    par = P.ctl[inst].parity;
-  }
-  Red red;
-  red.init();
-  bool listed = false;
-  if (live) limit_body<R, PHI, 0>(P, e, par, red, listed);
-  if (P.stage_idx == 0) {
-    if (live && red.tr) atomicAdd(&P.troubled_out[inst], red.tr);
-  } else {
-    block_commit<BS>(red, live, inst, P.acc, 3, P.stage_idx - 1);
+// Reductions of an element the limiters leave as it is: the stage's minima
+// and, in stage 3, its CFL step.
+__device__ __forceinline__ void limit_keep(const LimitParams& P, int e, double rmin, double pmin, Red& red) {
+  red.kr = dkey(rmin);
+  red.kp = dkey(pmin);
+  if (P.stage_idx == 3) {
+    const double d = P.m.dt_geo[e] / P.aux[2 * P.m.ld + e];
+    red.kd = dkey(d);
+    if (d != d) red.fl |= FLAG_NAN_DT;
   }
 }
 
-// The same limiter in two passes. The scan runs the detection for every
-// element with few registers, commits the minima (and CFL step) of the
-// elements the limiters leave as they are, and lists the others (troubled,
-// or below the positivity floor: a small minority); the rewrite pass then
-// runs the full reconstruction and positivity scaling on the listed
-// elements only, committing their minima one element at a time. Same
-// arithmetic, same results as limit_kernel.
-// The scan of the elements e0 .. e0 + BS - 1 by a block of BS threads.
-template <typename R, int PHI, int BS>
-__device__ __forceinline__ void limit_scan_body(const LimitParams& P, const int e0) {
-  const CfdMesh& m = P.m;
-  const int e = e0 + threadIdx.x;
-  bool live = e < m.num_elements;
-  int inst = 0;
-  if (live && m.instance) inst = m.instance[e];
-  if (inst < 0) {
-    live = false;
-    inst = 0;
-  }
-  int par = 0;
-  if (live && P.ctl) {
-    live = P.ctl[inst].status == CFD_RUN_ACTIVE;
-    par = P.ctl[inst].parity;
-  }
-  Red red;
-  red.init();
-  bool listed = false;
-  if (live) limit_body<R, PHI, 1>(P, e, par, red, listed);
-  warp_list_append(P.list, P.count, listed, e);
-  if (listed) red.init();
-  if (P.stage_idx == 0) {
-    if (live && red.tr) atomicAdd(&P.troubled_out[inst], red.tr);
-  } else {
-    block_commit<BS>(red, live && !listed, inst, P.acc, 3, P.stage_idx - 1);
-  }
-}
+constexpr int HALF = 16;  // lanes per element
 
-template <typename R, int PHI, int BS>
-__global__ void __launch_bounds__(BS) limit_scan_kernel(const LimitParams P) {
-  limit_scan_body<R, PHI, BS>(P, blockIdx.x * BS);
-}
-
-// The rewrite of one listed element by the four lanes base .. base + 3 of a
-// warp, lane c owning conserved variable c; the same results, bit for bit,
-// as limit_body's rewrite (PART 2). The detection and the troubled-cell
-// reconstruction run per variable in limit_body's operation order. The
-// positivity limiter and the element statistics deal node i out to lane
-// i % 4 (each lane gathers the node's four values by shuffles): the node
-// tests and the 60-step bisections then run four at a time, and their
-// results are combined by order-independent reductions (min / max, and for
-// the critical node the smallest index attaining the minimum theta, as the
-// sequential loop finds it). The element's reductions end in lane c = 0.
-template <typename R, int PHI>
-__device__ __forceinline__ void limit_rewrite_quad(const LimitParams& P, int e, int par, int c, unsigned qmask,
-                                                   int base, Red& red) {
-  const CfdMesh& m = P.m;
-  const int ld = m.ld;
-  R* __restrict__ q;
-  if (P.stage_idx == 0) {
-    q = (R*)P.q_io;
-  } else if (P.stage_idx == 2) {
-    q = (R*)P.stage;
-  } else {
-    q = (R*)(par ? P.x0 : P.x1);
-  }
-  const double gm1 = P.gamma - 1.0;
-  double a[4];
+// Zhang-Shu positivity scaling (limiting.py:166-200) of one element toward its
+// average by a half warp, lane t holding node i = min(t, 14)'s values v: density
+// scaling, then pressure scaling by the smallest theta of the nodes below the
+// target pt. Returns that theta (1 where none is) and its node.
+template <typename R>
+__device__ __forceinline__ void half_warp_positivity(R (&v)[4], const double a[4], double eps, double pt, double gm1,
+                                                     int i, unsigned hmask, double& th, int& node) {
+  if (__any_sync(hmask, (double)v[0] < eps)) {
+    double rmin = (double)v[0];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) a[k] = P.avg[k * ld + e];
-  const double pa = pressure_x(a[0], a[1], a[2], a[3], gm1);
-  const double eps = jmin(POSITIVITY_FLOOR, jmin(a[0], pa));
-  const double pt = pressure_target<R>(eps, pa, a[3], gm1);
-  const double det_tol = sizeof(R) == 8 ? DETECTION_TOLERANCE : DETECTION_TOLERANCE_FP32;
-  const int finfo = m.face_info[e];
-  bool troubled = false;
-  R scaled[3][4];
-  if (PHI != LIM_UNLIMITED) troubled = limit_detect<R, PHI>(P, e, q, a, finfo, det_tol, scaled);
-  const double rmin0 = P.aux[e], pmin0 = P.aux[ld + e];
-  const bool need_pos = (rmin0 < eps) || (pmin0 < pt);
-  if (!troubled && !need_pos) {  // (the scan lists no such element)
-    if (c == 0) {
-      red.kr = dkey(rmin0);
-      red.kp = dkey(pmin0);
-      if (P.stage_idx == 3) {
-        const double d = m.dt_geo[e] / P.aux[2 * ld + e];
-        red.kd = dkey(d);
-        if (d != d) red.fl |= FLAG_NAN_DT;
-      }
-    }
-    return;
-  }
-  const double ac_d = c == 0 ? a[0] : (c == 1 ? a[1] : (c == 2 ? a[2] : a[3]));
-  R s[NP];
+    for (int o = 1; o < HALF; o <<= 1) rmin = jmin(rmin, __shfl_xor_sync(hmask, rmin, o));
+    if (rmin < eps) {  // (a NaN among the nodes leaves the element as it is)
+      const double span = xsub(a[0], rmin);
+      const double theta = jmin(jmax(xdiv(xsub(a[0], eps), span), 0.0), 1.0);
 #pragma unroll
-  for (int i = 0; i < NP; ++i) s[i] = q[(c * NP + i) * ld + e];
-  if (troubled) {
-    // P1 midpoint values, phi-limited deltas, +/- rescaling, linear rebuild
-    // (limiting.py:153-162), in NumPy's operation order, for variable c
-    const R ac = (R)ac_d;
-    R deltas[3];
-    R pos = R(0), neg = R(0);
-#pragma unroll
-    for (int f = 0; f < 3; ++f) {
-      const R sc = c == 0 ? scaled[f][0] : (c == 1 ? scaled[f][1] : (c == 2 ? scaled[f][2] : scaled[f][3]));
-      R pr = xmul((R)tab::P1MID[f][0], s[0]);
-#pragma unroll
-      for (int i = 1; i < NP; ++i) pr = xadd(pr, xmul((R)tab::P1MID[f][i], s[i]));
-      pr = xsub(pr, ac);
-      R d = R(0);
-      if (pr != R(0)) d = xmul(pr, jmin(R(1), phi<R, PHI>(xdiv(sc, pr))));
-      deltas[f] = d;
-      pos = f == 0 ? jmax(d, R(0)) : xadd(pos, jmax(d, R(0)));
-      neg = f == 0 ? jmax(-d, R(0)) : xadd(neg, jmax(-d, R(0)));
-    }
-    const R thp = pos > R(0) ? jmin(R(1), xdiv(neg, pos)) : R(0);
-    const R thn = neg > R(0) ? jmin(R(1), xdiv(pos, neg)) : R(0);
-#pragma unroll
-    for (int f = 0; f < 3; ++f) deltas[f] = xsub(xmul(thp, jmax(deltas[f], R(0))), xmul(thn, jmax(-deltas[f], R(0))));
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      R v = xmul((R)tab::LINBASIS[i][0], deltas[0]);
-      v = xadd(v, xmul((R)tab::LINBASIS[i][1], deltas[1]));
-      v = xadd(v, xmul((R)tab::LINBASIS[i][2], deltas[2]));
-      s[i] = xadd(ac, v);
-    }
-    red.tr = c == 0 ? 1 : 0;
-  }
-  // ---- positivity (positivity() in common.cuh): density scaling
-  double rmin = (double)s[0];
-#pragma unroll
-  for (int i = 1; i < NP; ++i) rmin = jmin(rmin, (double)s[i]);
-  rmin = __shfl_sync(qmask, rmin, base);  // lane 0 holds the density
-  if (rmin < eps) {
-    const double span = xsub(a[0], rmin);
-    const double theta = jmin(jmax(xdiv(xsub(a[0], eps), span), 0.0), 1.0);
-#pragma unroll
-    for (int i = 0; i < NP; ++i) s[i] = (R)xadd(ac_d, xmul(theta, xsub((double)s[i], ac_d)));
-  }
-  // node tests: lane i % 4 tests node i and keeps its four values for the bisection
-  R keep[4][4];
-  unsigned need = 0;
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    R v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(qmask, s[i], base + k);
-    if ((i & 3) == c) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) keep[i >> 2][k] = v[k];
-      if (pressure_near(v[0], v[1], v[2], v[3], gm1, pt) < pt) need |= 1u << i;
+      for (int k = 0; k < 4; ++k) v[k] = (R)xadd(a[k], xmul(theta, xsub((double)v[k], a[k])));
     }
   }
-  need |= __shfl_xor_sync(qmask, need, 1);
-  need |= __shfl_xor_sync(qmask, need, 2);
-  double th = 1.0;
-  int node = -1;
-  if (need) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = 4 * k + c;
-      if (i >= NP || !((need >> i) & 1u)) continue;
-      const double d0 = xsub((double)keep[k][0], a[0]), d1 = xsub((double)keep[k][1], a[1]);
-      const double d2 = xsub((double)keep[k][2], a[2]), d3 = xsub((double)keep[k][3], a[3]);
-      double lo = 0.0, hi = 1.0;
-#pragma unroll 1
-      for (int it = 0; it < BISECTION_STEPS; ++it) {
-        const double mid = xmul(0.5, xadd(lo, hi));
-        const bool ok = pressure_x(xadd(a[0], xmul(mid, d0)), xadd(a[1], xmul(mid, d1)), xadd(a[2], xmul(mid, d2)),
-                                   xadd(a[3], xmul(mid, d3)), gm1) >= pt;
-        lo = ok ? mid : lo;
-        hi = ok ? hi : mid;
-      }
-      if (lo < th) {  // ascending i within the lane: the smallest index of a tie stays
+  const bool low = pressure_near(v[0], v[1], v[2], v[3], gm1, pt) < pt;
+  th = 1.0;
+  node = -1;
+  if (__any_sync(hmask, low)) {
+    if (low) {
+      const double lo = pressure_theta(a, xsub((double)v[0], a[0]), xsub((double)v[1], a[1]),
+                                       xsub((double)v[2], a[2]), xsub((double)v[3], a[3]), gm1, pt);
+      if (lo < th) {
         th = lo;
         node = i;
       }
     }
+    __syncwarp(hmask);
 #pragma unroll
-    for (int off = 1; off <= 2; off <<= 1) {
-      const double oth = __shfl_xor_sync(qmask, th, off);
-      const int onode = __shfl_xor_sync(qmask, node, off);
+    for (int o = 1; o < HALF; o <<= 1) {
+      const double oth = __shfl_xor_sync(hmask, th, o);
+      const int onode = __shfl_xor_sync(hmask, node, o);
       if (oth < th || (oth == th && onode >= 0 && (node < 0 || onode < node))) {
         th = oth;
         node = onode;
@@ -417,82 +84,321 @@ __device__ __forceinline__ void limit_rewrite_quad(const LimitParams& P, int e, 
     }
     if (th < 1.0) {
 #pragma unroll
-      for (int i = 0; i < NP; ++i) s[i] = (R)xadd(ac_d, xmul(th, xsub((double)s[i], ac_d)));
+      for (int k = 0; k < 4; ++k) v[k] = (R)xadd(a[k], xmul(th, xsub((double)v[k], a[k])));
     }
   }
-  if (P.pos_out && c == 0) {
+}
+
+// The scan of one element: the troubled-cell test (limiting.py:128-151: the
+// scaled neighbour differences from Cockburn-Shu coefficients and neighbour or
+// ghost averages, and whether a density or energy trace at a face midpoint
+// leaves its minmod bound) and the positivity test on the stage's nodal
+// minima. An element the limiters leave as it is contributes its minima (and
+// CFL step) to `red`; any other is `listed` for limit_half_warp. Writes the
+// troubled flag where asked for.
+//
+// Bound by memory latency on large meshes (10 of 15 cycles between two
+// instructions of a warp went to loads): every load but the neighbours'
+// averages is therefore issued before the first value is used, the loop
+// state's among them, so that an element takes two round trips.
+template <typename R, int PHI>
+__device__ __forceinline__ bool limit_scan_one(const LimitParams& P, int e, int inst, Red& red) {
+  const CfdMesh& m = P.m;
+  const int ld = m.ld;
+  const volatile CfdControl* ctl = P.ctl ? P.ctl + inst : nullptr;
+  const int status = ctl ? ctl->status : CFD_RUN_ACTIVE, par = ctl ? ctl->parity : 0;
+  const double rmin0 = P.aux[e], pmin0 = P.aux[ld + e];
+  double a[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) a[c] = P.avg[c * ld + e];
+  int finfo = 0, nb[3] = {0, 0, 0};
+  R co[6] = {}, tr[3][2] = {};
+  if (PHI != LIM_UNLIMITED) {
+    finfo = m.face_info[e];
+    const R* __restrict__ cs = GeoPtr<R>::cs(m);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) nb[f] = m.neighbor[f * ld + e];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) co[k] = cs[k * ld + e];
+    const R* __restrict__ q = limit_state<R>(P, par);
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) tr[f][k] = q[(3 * k * NP + tab::MID_NODES[f]) * ld + e];
+  }
+  if (status != CFD_RUN_ACTIVE) return false;
+  bool troubled = false;
+  if (PHI != LIM_UNLIMITED) {
+    R diff[3][2];  // density and energy: the detection components
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const int kind = (finfo >> (8 * f)) & 3;
+      double na[2];
+      if (kind == CFD_FACE_INTERIOR) {
+        na[0] = P.avg[nb[f]];
+        na[1] = P.avg[3 * ld + nb[f]];
+      } else if (kind == CFD_FACE_SLIP_WALL) {  // the mirror keeps both
+        na[0] = a[0];
+        na[1] = a[3];
+      } else {
+        // the ghost average: the fixed state, or the exact state's row after its node rows
+        const int row = nb[f] + (kind == CFD_FACE_EXACT_STATE ? NFP : 0);
+        na[0] = m.bc_states[row * 4];
+        na[1] = m.bc_states[row * 4 + 3];
+      }
+      diff[f][0] = (R)xsub(na[0], a[0]);
+      diff[f][1] = (R)xsub(na[1], a[3]);
+    }
+    const double det_tol = sizeof(R) == 8 ? DETECTION_TOLERANCE : DETECTION_TOLERANCE_FP32;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const int pf = (finfo >> (8 * f + 4)) & 3;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const double ac = k == 0 ? a[0] : a[3];
+        const R pd = pf == 0 ? diff[0][k] : (pf == 1 ? diff[1][k] : diff[2][k]);
+        const R sc = xmul((R)NEIGHBOR_FACTOR, xadd(xmul(co[f], diff[f][k]), xmul(co[3 + f], pd)));
+        const R t = xsub(tr[f][k], (R)ac);
+        troubled |= (double)abs_(xsub(minmod2(t, sc), t)) > xmul(det_tol, fabs(ac));
+      }
+    }
+  }
+  if (P.flags) P.flags[e] = troubled ? 1 : 0;
+  const double gm1 = P.gamma - 1.0;
+  const double pa = pressure_x(a[0], a[1], a[2], a[3], gm1);
+  const double eps = jmin(POSITIVITY_FLOOR, jmin(a[0], pa));
+  const double pt = pressure_target<R>(eps, pa, a[3], gm1);
+  if (troubled || rmin0 < eps || pmin0 < pt) return true;
+  limit_keep(P, e, rmin0, pmin0, red);
+  return false;
+}
+
+// The limiters on element e by the sixteen lanes of a half warp: troubled-cell
+// test, reconstruction (limiting.py:136-163) and positivity scaling
+// (limiting.py:166-200), in place on the stage state. Every value is formed in
+// NumPy's operation order, whichever lane forms it:
+//   lane t < 12 owns (face f = t / 4, variable c = t % 4): the scaled
+//     neighbour difference, its test, the P1 midpoint value (one sequential sum
+//     over the nodes) and its limited delta;
+//   lane t < 15 owns node t: the rebuilt state, the positivity scalings, the
+//     bisection of its pressure and its statistics (lane 15 repeats node 14).
+// Theta and its critical node (the smallest index attaining the minimum, as a
+// sequential loop finds it) are order-independent reductions over the lanes;
+// each lane's `red` takes its own node.
+//
+// What bounds this pass is the serial chain of one element, not the count of
+// elements: on a shock tube a few hundred of them are rewritten per stage. With
+// four lanes an element, one variable each, the node tests and statistics ran
+// one node after the other in the warp (15 double divisions, reciprocals and
+// square roots in a row): 18.5 us for the 2,000-element tube and 77 us for a
+// 40,000-element channel in FP64, at 15 % of the issue slots; a lane per node
+// does them at once.
+template <typename R> struct LimitShared {
+  R v[NP * 4];  // the element's nodal values, [node][variable]
+  R d[12];      // limited deltas, [face][variable]
+};
+
+template <typename R, int PHI>
+__device__ __forceinline__ void limit_half_warp(const LimitParams& P, int e, int inst, int t, unsigned hmask, int base,
+                                                LimitShared<R>& sm, bool scanned, Red& red) {
+  const CfdMesh& m = P.m;
+  const int ld = m.ld;
+  const volatile CfdControl* ctl = P.ctl ? P.ctl + inst : nullptr;
+  const int status = ctl ? ctl->status : CFD_RUN_ACTIVE, par = ctl ? ctl->parity : 0;
+  R* __restrict__ q = limit_state<R>(P, par);
+  const double gm1 = P.gamma - 1.0;
+  const int i = t < NP ? t : NP - 1;
+  const int finfo = m.face_info[e];
+  double a[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) a[k] = P.avg[k * ld + e];
+  const double rmin0 = P.aux[e], pmin0 = P.aux[ld + e];
+  const int f = t < 12 ? t >> 2 : 0, c = t & 3;
+  const int nb_ = m.neighbor[f * ld + e];
+  R v[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) v[c] = q[(c * NP + i) * ld + e];
+  if (status != CFD_RUN_ACTIVE) return;  // a finished instance
+  const double ac_d = c == 0 ? a[0] : (c == 1 ? a[1] : (c == 2 ? a[2] : a[3]));
+  const R ac = (R)ac_d;
+  bool troubled = false;
+  R sc = R(0);
+  if (PHI != LIM_UNLIMITED) {
+    // the scaled neighbour difference of (f, c), as limit_scan_one forms it
+    const int kind = (finfo >> (8 * f)) & 3, pf = (finfo >> (8 * f + 4)) & 3;
+    const int nb = nb_;
+    const R* __restrict__ cs = GeoPtr<R>::cs(m);
+    const R al = cs[f * ld + e], be = cs[(3 + f) * ld + e];
+    double na;
+    if (kind == CFD_FACE_INTERIOR) {
+      na = P.avg[c * ld + nb];
+    } else if (kind == CFD_FACE_SLIP_WALL) {
+      const double nx = m.face_geo[(3 * f) * ld + e], ny = m.face_geo[(3 * f + 1) * ld + e];
+      const double mn = xadd(xmul(a[1], nx), xmul(a[2], ny));
+      na = (c == 0 || c == 3) ? ac_d : xsub(ac_d, xmul(xmul(2.0, mn), c == 1 ? nx : ny));
+    } else {
+      na = m.bc_states[(nb + (kind == CFD_FACE_EXACT_STATE ? NFP : 0)) * 4 + c];
+    }
+    const R diff = (R)xsub(na, ac_d);
+    const R pd = __shfl_sync(hmask, diff, base + 4 * pf + c);
+    sc = xmul((R)NEIGHBOR_FACTOR, xadd(xmul(al, diff), xmul(be, pd)));
+    if (t < NP) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sm.v[4 * t + k] = v[k];
+    }
+    __syncwarp(hmask);
+    const double det_tol = sizeof(R) == 8 ? DETECTION_TOLERANCE : DETECTION_TOLERANCE_FP32;
+    const int mid = f == 0 ? tab::MID_NODES[0] : (f == 1 ? tab::MID_NODES[1] : tab::MID_NODES[2]);
+    const R tr = xsub(sm.v[4 * mid + c], ac);
+    const R ex = abs_(xsub(minmod2(tr, sc), tr));
+    troubled = __any_sync(hmask, t < 12 && (c == 0 || c == 3) && (double)ex > xmul(det_tol, fabs(ac_d)));
+  }
+  if (!scanned && P.flags && t == 0) P.flags[e] = troubled ? 1 : 0;
+  const double pa = pressure_x(a[0], a[1], a[2], a[3], gm1);
+  const double eps = jmin(POSITIVITY_FLOOR, jmin(a[0], pa));
+  const double pt = pressure_target<R>(eps, pa, a[3], gm1);
+  const bool need_pos = (rmin0 < eps) || (pmin0 < pt);
+  if (!troubled && !need_pos) {
+    if (t == 0) limit_keep(P, e, rmin0, pmin0, red);
+    return;
+  }
+  if (troubled) {
+    // P1 midpoint values, phi-limited deltas, +/- rescaling, linear rebuild (limiting.py:153-162)
+    const double* __restrict__ row = tab::P1MID[f];
+    R pr = xmul((R)row[0], sm.v[c]);
+#pragma unroll
+    for (int j = 1; j < NP; ++j) pr = xadd(pr, xmul((R)row[j], sm.v[4 * j + c]));
+    pr = xsub(pr, ac);
+    R d = R(0);
+    if (pr != R(0)) d = xmul(pr, jmin(R(1), phi<R, PHI>(xdiv(sc, pr))));
+    const R d0 = __shfl_sync(hmask, d, base + c), d1 = __shfl_sync(hmask, d, base + 4 + c);
+    const R d2 = __shfl_sync(hmask, d, base + 8 + c);
+    const R pos = xadd(xadd(jmax(d0, R(0)), jmax(d1, R(0))), jmax(d2, R(0)));
+    const R neg = xadd(xadd(jmax(-d0, R(0)), jmax(-d1, R(0))), jmax(-d2, R(0)));
+    const R thp = pos > R(0) ? jmin(R(1), xdiv(neg, pos)) : R(0);
+    const R thn = neg > R(0) ? jmin(R(1), xdiv(pos, neg)) : R(0);
+    if (t < 12) sm.d[t] = xsub(xmul(thp, jmax(d, R(0))), xmul(thn, jmax(-d, R(0))));
+    __syncwarp(hmask);
+    const R l0 = (R)tab::LINBASIS[i][0], l1 = (R)tab::LINBASIS[i][1], l2 = (R)tab::LINBASIS[i][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      R x = xmul(l0, sm.d[k]);
+      x = xadd(x, xmul(l1, sm.d[4 + k]));
+      x = xadd(x, xmul(l2, sm.d[8 + k]));
+      v[k] = xadd((R)a[k], x);
+    }
+    if (t == 0) red.tr += 1;
+  }
+  double th;
+  int node;
+  half_warp_positivity<R>(v, a, eps, pt, gm1, i, hmask, th, node);
+  if (P.pos_out && t == 0) {
     P.pos_out[e] = th;
     P.pos_out[ld + e] = (double)node;
   }
+  if (t < NP) {
 #pragma unroll
-  for (int i = 0; i < NP; ++i) q[(c * NP + i) * ld + e] = s[i];
-  // ---- element statistics (element_stats in common.cuh), node i in lane i % 4
-  double rmn = INFINITY, pmn = INFINITY, lam = -INFINITY;
-  bool finite = true, lam_nan = false;
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    R v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(qmask, s[i], base + k);
-    if ((i & 3) == c) {
-      const double p = node_pressure<R>(v[0], v[1], v[2], v[3], gm1, POSITIVITY_FLOOR);
-      rmn = fmin(rmn, (double)v[0]);
-      pmn = fmin(pmn, p);
-      const double sp = wave_speed<R>(v[0], v[1], v[2], v[3], P.gamma);
-      lam_nan |= (sp != sp);
-      lam = fmax(lam, sp);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) finite &= finite_(v[k]);
-    }
+    for (int k = 0; k < 4; ++k) q[(k * NP + t) * ld + e] = v[k];
   }
-  unsigned bits = (finite ? 1u : 0u) | (lam_nan ? 2u : 0u);
-#pragma unroll
-  for (int off = 1; off <= 2; off <<= 1) {
-    rmn = fmin(rmn, __shfl_xor_sync(qmask, rmn, off));
-    pmn = fmin(pmn, __shfl_xor_sync(qmask, pmn, off));
-    lam = fmax(lam, __shfl_xor_sync(qmask, lam, off));
-    const unsigned ob = __shfl_xor_sync(qmask, bits, off);
-    bits = ((bits & ob) & 1u) | ((bits | ob) & 2u);
+  // ---- statistics of the own node (element_stats in common.cuh); the wave
+  // speed only where the CFL step is formed. The minima of the element are left
+  // to the block's reduction: dt_geo / speed is monotone, so its least value
+  // over the nodes is that of the largest speed.
+  red.kr = min(red.kr, dkey(fmin(INFINITY, (double)v[0])));
+  red.kp = min(red.kp, dkey(fmin(INFINITY, node_pressure<R>(v[0], v[1], v[2], v[3], gm1, POSITIVITY_FLOOR))));
+  if (!(finite_(v[0]) && finite_(v[1]) && finite_(v[2]) && finite_(v[3]))) red.fl |= FLAG_NONFINITE;
+  if (P.stage_idx == 3) {
+    const double d = m.dt_geo[e] / wave_speed<R>(v[0], v[1], v[2], v[3], P.gamma);
+    if (d != d) red.fl |= FLAG_NAN_DT;
+    red.kd = min(red.kd, dkey(d));
   }
-  if (bits & 2u) lam = NAN;
-  if (c == 0) {
-    if (!(bits & 1u)) red.fl |= FLAG_NONFINITE;
-    red.kr = dkey(rmn);
-    red.kp = dkey(pmn);
-    if (P.stage_idx == 3) {
-      const double d = m.dt_geo[e] / lam;
-      red.kd = dkey(d);
-      if (d != d) red.fl |= FLAG_NAN_DT;
-    }
-  }
+  __syncwarp(hmask);  // the half warp's next element reuses sm
 }
 
-// The rewrite of the listed elements, four lanes per element, spread over
-// every thread of the grid (the block size is a multiple of 4, so the four
-// lanes of an element are always in one warp and take the same trips).
-template <typename R, int PHI>
-__device__ __forceinline__ void limit_rewrite_body(const LimitParams& P) {
+// The limiter on the elements e0 .. e0 + EPB - 1 by a block of BS threads.
+//   EPB = BS: every thread scans one element, the block lists those the
+//     limiters change in shared memory, and its BS / 16 half warps rewrite
+//     them. The averages the tests read are the stage's and change no more, so
+//     the rewrite needs no other block.
+//   EPB = BS / 16: each half warp takes one element directly, no list (smaller
+//     meshes, where the scan would only lengthen the chain).
+// The block reduces to one commit; an element of another instance than the
+// block's lowest live one (possible where instances are not aligned to blocks)
+// commits by itself.
+template <typename R, int PHI, int BS, int EPB>
+__device__ __forceinline__ void limit_block_body(const LimitParams& P, const int e0) {
+  constexpr bool SCAN = EPB > BS / HALF;
+  __shared__ LimitShared<R> s_half[BS / HALF];
+  __shared__ int s_list[SCAN ? EPB : 1];
+  __shared__ int s_count, s_inst;
   const CfdMesh& m = P.m;
-  const int n = *(volatile int*)P.count;
-  const int lane = threadIdx.x & 31, c = lane & 3, base = lane & ~3;
-  const unsigned qmask = 0xfu << base;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; t < n; t += (gridDim.x * blockDim.x) >> 2) {
-    const int e = P.list[t];
-    const int inst = m.instance ? m.instance[e] : 0;
-    const int par = P.ctl ? P.ctl[inst].parity : 0;
-    Red red;
-    red.init();
-    limit_rewrite_quad<R, PHI>(P, e, par, c, qmask, base, red);
-    if (c != 0) continue;
-    if (P.stage_idx == 0) {
-      if (red.tr) atomicAdd(&P.troubled_out[inst], red.tr);
-    } else {
-      commit_one(red, P.acc + 3 * inst + (P.stage_idx - 1));
+  const int lane = threadIdx.x & 31, t = lane & (HALF - 1), base = lane & HALF;
+  const unsigned hmask = 0xffffu << base;
+  LimitShared<R>& sm = s_half[threadIdx.x / HALF];
+  const int e = e0 + (SCAN ? (int)threadIdx.x : (int)threadIdx.x / HALF);
+  bool live = e < m.num_elements && (!SCAN || (int)threadIdx.x < EPB);
+  int inst = 0;
+  if (live && m.instance) inst = m.instance[e];
+  if (inst < 0) {  // padding between instances
+    live = false;
+    inst = 0;
+  }
+  if (threadIdx.x == 0) {
+    s_count = 0;
+    s_inst = 0x7fffffff;
+  }
+  __syncthreads();
+  if (live && m.instance) atomicMin(&s_inst, inst);
+  Red red, own;
+  red.init();
+  own.init();
+  if (SCAN) {
+    if (live && limit_scan_one<R, PHI>(P, e, inst, own)) s_list[atomicAdd(&s_count, 1)] = e;
+  } else {
+    if (live) limit_half_warp<R, PHI>(P, e, inst, t, hmask, base, sm, false, own);
+  }
+  __syncthreads();
+  const int inst0 = m.instance ? s_inst : 0;
+  auto take = [&](const Red& r, int i) {
+    if (i == inst0) red.merge(r);
+    else if (P.stage_idx != 0) commit_one(r, P.acc + 3 * i + (P.stage_idx - 1));
+    else if (r.tr) atomicAdd(&P.troubled_out[i], r.tr);
+  };
+  if (live) take(own, inst);
+  if (SCAN) {
+    for (int k = threadIdx.x / HALF; k < s_count; k += BS / HALF) {
+      const int le = s_list[k];
+      const int li = m.instance ? m.instance[le] : 0;
+      own.init();
+      limit_half_warp<R, PHI>(P, le, li, t, hmask, base, sm, true, own);
+      take(own, li);
     }
+  }
+  if (P.stage_idx == 0) {
+    const int n = __reduce_add_sync(0xffffffffu, red.tr);
+    if (lane == 0 && n) atomicAdd(&P.troubled_out[inst0], n);
+  } else if (inst0 != 0x7fffffff) {
+    commit_keys(red, P.acc + 3 * inst0 + (P.stage_idx - 1));
   }
 }
 
-template <typename R, int PHI>
-__global__ void __launch_bounds__(64) limit_rewrite_kernel(const LimitParams P) {
-  limit_rewrite_body<R, PHI>(P);
+constexpr int LIMIT_BS = 128;
+// Which form: one RK3 attempt (three stages, graph replay) with the same stage
+// kernel, us; the channel's elements are nearly all rewritten, the tube's few.
+//                                 two launches   direct   scan of 32   of 64   of 128
+//   tube,     2,000, FP64              136          104        -          -       -
+//   tube,    32,000, FP32              170           -         97         93      93
+//   channel, 10,000, FP64               -            -        138        173     218
+//   channel, 40,000, FP64              279           -        231        262     321
+//   tube,   800,000, FP64            3,373           -         -          -     3,236
+// (two launches: a scan of the whole mesh, then a rewrite of a global list.)
+// A block that rewrites all it scans takes EPB / 8 rounds of some 4,900 cycles,
+// so few elements a block balance better while the blocks fit the GPU at once
+// (seven of them an SM at 72 registers); the direct form adds nothing once its
+// blocks need more than one wave, and on large meshes the fixed work of a block
+// counts instead.
+constexpr int LIMIT_DIRECT_MAX = 5900, LIMIT_SCAN32_MAX = 70000;
+template <typename R, int PHI, int EPB>
+__global__ void __launch_bounds__(LIMIT_BS, 7) limit_kernel(const LimitParams P) {
+  limit_block_body<R, PHI, LIMIT_BS, EPB>(P, blockIdx.x * EPB);
 }

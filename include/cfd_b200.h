@@ -220,10 +220,9 @@ typedef struct CfdSolver {
                               12 / 13 as 9 with the volume node loop kept rolled ([Dr|Ds] from
                               the constant bank), with unrolled / rolled face rounds,
                               14 as 5 with the volume node loop kept rolled */
-    int32_t* limit_list;   /* optional [CFD_LIMIT_LIST_HEADER + ld] scratch: with it the limiter
-                              runs in two passes (a light detection pass over every element,
-                              then the rewrite of the troubled / non-positive ones only);
-                              NULL: one pass. cfd_rk3_begin resets its counters. */
+    int32_t* limit_list;   /* optional [CFD_LIMIT_LIST_HEADER + ld] scratch; the limiter lists the
+                              elements it rewrites per block and no longer uses it
+                              (cfd_batch_advance still asks for it) */
     uint8_t* troubled_flags; /* optional [3][ld]: the troubled-cell indicator of limiting.py:147-151
                               (1 = troubled, 0 = not) of every active element; stage k of an attempt
                               writes row k-1, cfd_limit writes row 0. NULL: not written. */
@@ -299,7 +298,7 @@ int cfd_run_control(const CfdSolver* s, void* stream);
  * tiles of all instances, with a grid-wide barrier between the phases of an
  * attempt (zero the reduction slots; stage k and its limiter passes for
  * k = 1, 2, 3; report and control). Returns early once no instance is active.
- * Needs the limit_list scratch (the limiter runs in its two-pass form). The
+ * Needs the limit_list scratch. The
  * tile shape is fixed per precision (FP32: variant 9, FP64: variant 3) and the
  * per-element arithmetic is that of the separate launches, so the results
  * equal those of `attempts` x (cfd_rk3_attempt + cfd_run_control) with that
