@@ -1,9 +1,10 @@
 """Autotuner of the stage-kernel shape (elements per block, tile staging).
 
 The fused stage kernel comes in these shapes (CfdSolver.variant):
-  0  tiled, 32 elements (64 threads) per block, state and geometry staged in
-     shared memory, stage base read from global memory in the epilogue
-  1  tiled, 32 elements per block, stage base staged in shared memory too
+  0  chosen by the library from the mesh's size: one thread per node on small
+     meshes, the tile shape that is usually fastest on larger ones
+  1  tiled, 32 elements (64 threads) per block, state, geometry and stage base
+     staged in shared memory
   2  register-only pair kernel (block size 64/128/256 threads)
   3  tiled, 64 elements (128 threads) per block
   4  tiled, 32 elements per block, registers capped so that 10 (FP32) / 8

@@ -189,6 +189,9 @@ class BatchedEulerSolver:
                                  persistent=self.persistent, compact=self.compact,
                                  _parts=[self._parts[i] for i in keep])
         sub._struct.block_size = self._struct.block_size
+        # one instance left is still a batch: variant 0 then keeps the batch's
+        # FP64 kernel, whose results another one may round differently
+        sub._struct.mesh.flags |= 1
         raw = bytearray()
         for k, i in enumerate(keep):
             c = _native.CfdControl.from_buffer_copy(bytes(ctl[i]))

@@ -483,6 +483,7 @@ __device__ __forceinline__ R stage3_combine(R b, R v) {
 #include "stage_pair.cuh"
 #include "stage_tile.cuh"
 #include "limiter.cuh"
+#include "stage_node.cuh"
 #include "control.cuh"
 #include "batch.cuh"
 
@@ -527,6 +528,31 @@ void launch_tile(const StageParams& p, cudaStream_t st) {
   const unsigned g = blocks_for(p.m.num_elements, EPB);
   stage_tile_kernel<R, FLUX, MODE, EPB, SB, MINB, UF, PACK, CALL, FJ, VR><<<g, 2 * EPB, L::BYTES, st>>>(p);
 }
+// Variant 0, by size. One thread per node up to NODE_MAX elements, and on meshes
+// whose leading dimension does not keep the tiled kernels' 16-byte copies
+// aligned and inside a row; above, tiles of 32 elements, in FP64 of 64 elements
+// from TILE64_MIN on. One RK3 attempt (graph replay), us:
+//   elements                  one thread per node   tiles of 32   tiles of 64
+//   2,000    FP64 / FP32            48 /  41          107 /  62     112 /  61
+//   8,000    FP64 / FP32           102 /  70          105 /  71     105 /  67
+//   32,000   FP64 / FP32           330 / 160          213 / 106     244 / 101
+//   128,000  FP64                       -                 655           560
+//   1.05 M   FP64 / FP32                -          3,080 / 1,432   2,903 / 1,290
+// In FP32-mixed the node form rounds as tiles of 32 do (but for a few sums in
+// the limited stages); tiles of 64 with the flux as a call round more of them
+// differently, which a run near the limiter's thresholds shows, so that choice
+// is left to the autotuner. A batch (flags bit 0) keeps one
+// FP64 kernel at every size, because it may be repacked into a smaller one.
+constexpr int NODE_MAX = 8000, TILE64_MIN = 100000;
+template <typename R, int FLUX, int MODE>
+void launch_stage_default(const StageParams& p, cudaStream_t st) {
+  const int n = p.m.num_elements;
+  const bool batch = p.m.flags & 1;
+  if (p.m.ld % 64 || (n <= NODE_MAX && !(batch && sizeof(R) == 8)))
+    stage_node_kernel<R, FLUX, MODE><<<blocks_for(n, NODE_EPB), NODE_BS, 0, st>>>(p);
+  else if (sizeof(R) == 8 && n >= TILE64_MIN && !batch) launch_tile<R, FLUX, MODE, 64, false, 3, false>(p, st);
+  else launch_tile<R, FLUX, MODE, 32, false>(p, st);
+}
 template <typename R, int FLUX, int MODE>
 void launch_stage_variant(const StageParams& p, int variant, int bs, cudaStream_t st) {
   if (variant == 2) launch_stage_bs<R, FLUX, MODE>(p, bs, st);
@@ -551,7 +577,7 @@ void launch_stage_variant(const StageParams& p, int variant, int bs, cudaStream_
     launch_tile<R, FLUX, MODE, 64, true, (sizeof(R) == 4 ? 512 : 384) / 128, false, true, true, false, true>(p, st);
   else if (variant == 14)
     launch_tile<R, FLUX, MODE, 64, false, (sizeof(R) == 4 ? 512 : 384) / 128, false, true, false, false, true>(p, st);
-  else launch_tile<R, FLUX, MODE, 32, false>(p, st);
+  else launch_stage_default<R, FLUX, MODE>(p, st);
 }
 // One precision and mode of the stage kernels, every flux and shape; each
 // combination is instantiated in its own object (stage_inst.cu).

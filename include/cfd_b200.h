@@ -206,7 +206,9 @@ typedef struct CfdSolver {
     CfdStepReport* report; /* [num_instances] */
     CfdControl* control;   /* [num_instances] */
     int32_t block_size;    /* threads per block of the pair stage kernel (64, 128, 256); 0 = default */
-    int32_t variant;       /* stage kernel: 0 tiled (default), 1 tiled + staged base rows,
+    int32_t variant;       /* stage kernel: 0 chosen by the size of the mesh (default: one thread per
+                              node on small meshes, else a tiled shape), 1 tiled (32 elements per
+                              block) + staged base rows,
                               2 register-only pair kernel, 3 tiled with 64 elements per block,
                               4 tiled with registers capped for more resident blocks,
                               5 tiled with 64 elements per block and the face rounds kept rolled,
