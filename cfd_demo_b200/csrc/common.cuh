@@ -484,6 +484,7 @@ __device__ __forceinline__ R stage3_combine(R b, R v) {
 #include "stage_tile.cuh"
 #include "limiter.cuh"
 #include "stage_node.cuh"
+#include "stage_quad.cuh"
 #include "control.cuh"
 #include "batch.cuh"
 
@@ -528,29 +529,46 @@ void launch_tile(const StageParams& p, cudaStream_t st) {
   const unsigned g = blocks_for(p.m.num_elements, EPB);
   stage_tile_kernel<R, FLUX, MODE, EPB, SB, MINB, UF, PACK, CALL, FJ, VR><<<g, 2 * EPB, L::BYTES, st>>>(p);
 }
+template <int FLUX, int MODE>
+void launch_quad(const StageParams& p, cudaStream_t st) {
+  constexpr int BYTES = (int)sizeof(QuadShared) * (QUAD_BS / 32);
+  constexpr int MAX_DEV = 64;  // the > 48 KB opt-in, once per instantiation and device (as launch_tile)
+  static bool configured[MAX_DEV] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= MAX_DEV || !configured[dev]) {
+    cudaFuncSetAttribute(stage_quad_kernel<FLUX, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+    if (dev >= 0 && dev < MAX_DEV) configured[dev] = true;
+  }
+  stage_quad_kernel<FLUX, MODE><<<blocks_for(p.m.num_elements, QUAD_EPB), QUAD_BS, BYTES, st>>>(p);
+}
 // Variant 0, by size. One thread per node up to NODE_MAX elements, and on meshes
-// whose leading dimension does not keep the tiled kernels' 16-byte copies
-// aligned and inside a row; above, tiles of 32 elements, in FP64 of 64 elements
-// from TILE64_MIN on. One RK3 attempt (graph replay), us:
-//   elements                  one thread per node   tiles of 32   tiles of 64
-//   2,000    FP64 / FP32            48 /  41          107 /  62     112 /  61
-//   8,000    FP64 / FP32           102 /  70          105 /  71     105 /  67
-//   32,000   FP64 / FP32           330 / 160          213 / 106     244 / 101
-//   128,000  FP64                       -                 655           560
-//   1.05 M   FP64 / FP32                -          3,080 / 1,432   2,903 / 1,290
+// whose leading dimension does not keep the other forms' 16-byte copies aligned
+// and inside a row; above, four lanes per element in FP64 and tiles of 32
+// elements in FP32-mixed. One RK3 attempt (graph replay), us (larger meshes:
+// stage_quad.cuh):
+//   elements                  one thread per node   four lanes   tiles of 32   tiles of 64
+//   2,000    FP64 / FP32            48 /  41             -         107 /  62     112 /  61
+//   8,000    FP64 / FP32           102 /  70            98         105 /  71     105 /  67
+//   32,000   FP64 / FP32           330 / 160           167         213 / 106     237 / 101
+//   1.05 M   FP32                                                  1,432         1,290
 // In FP32-mixed the node form rounds as tiles of 32 do (but for a few sums in
 // the limited stages); tiles of 64 with the flux as a call round more of them
 // differently, which a run near the limiter's thresholds shows, so that choice
-// is left to the autotuner. A batch (flags bit 0) keeps one
-// FP64 kernel at every size, because it may be repacked into a smaller one.
-constexpr int NODE_MAX = 8000, TILE64_MIN = 100000;
+// is left to the autotuner. A batch (flags bit 0) keeps one FP64 kernel at every
+// size, because it may be repacked into a smaller one.
+constexpr int NODE_MAX = 8000;
+// The differentiable step's shape behind variant 0, at every size: tiles of 32.
+// Its gradient takes the branch of |u.n| and of the limiter that round-off picks
+// where a region is uniform, so a kernel that rounds differently would change
+// the gradient there (1.9e-4 of its norm on a shock tube), not its last bits.
+constexpr int SHAPE_TILE32 = -1;
 template <typename R, int FLUX, int MODE>
 void launch_stage_default(const StageParams& p, cudaStream_t st) {
   const int n = p.m.num_elements;
-  const bool batch = p.m.flags & 1;
-  if (p.m.ld % 64 || (n <= NODE_MAX && !(batch && sizeof(R) == 8)))
+  if (p.m.ld % 64 || (n <= NODE_MAX && !(sizeof(R) == 8 && (p.m.flags & 1))))
     stage_node_kernel<R, FLUX, MODE><<<blocks_for(n, NODE_EPB), NODE_BS, 0, st>>>(p);
-  else if (sizeof(R) == 8 && n >= TILE64_MIN && !batch) launch_tile<R, FLUX, MODE, 64, false, 3, false>(p, st);
+  else if constexpr (sizeof(R) == 8) launch_quad<FLUX, MODE>(p, st);
   else launch_tile<R, FLUX, MODE, 32, false>(p, st);
 }
 template <typename R, int FLUX, int MODE>
@@ -577,6 +595,7 @@ void launch_stage_variant(const StageParams& p, int variant, int bs, cudaStream_
     launch_tile<R, FLUX, MODE, 64, true, (sizeof(R) == 4 ? 512 : 384) / 128, false, true, true, false, true>(p, st);
   else if (variant == 14)
     launch_tile<R, FLUX, MODE, 64, false, (sizeof(R) == 4 ? 512 : 384) / 128, false, true, false, false, true>(p, st);
+  else if (variant == SHAPE_TILE32) launch_tile<R, FLUX, MODE, 32, false>(p, st);
   else launch_stage_default<R, FLUX, MODE>(p, st);
 }
 // One precision and mode of the stage kernels, every flux and shape; each

@@ -731,7 +731,7 @@ int cfd_rk3_step_fixed(const CfdSolver* s, const void* q_in, void* q_out, void* 
   // into the tape as it goes (the register-only pair kernel cannot copy its
   // input), and the averages / minima / positivity theta land there directly
   CfdSolver sv = *s;
-  if (tape && sv.variant == 2) sv.variant = 0;
+  if (sv.variant == 0 || (tape && sv.variant == 2)) sv.variant = SHAPE_TILE32;
   for (int k = 1; k <= 3; ++k) {
     StageParams p;
     memset(&p, 0, sizeof(p));

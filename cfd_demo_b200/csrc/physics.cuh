@@ -65,16 +65,20 @@ template <typename R> struct Prim {
   R rho, u, v, p, inv_rho;
 };
 
-// euler.py:21-27
+// euler.py:21-27, from the reciprocal of the density
 template <typename R>
-__device__ __forceinline__ Prim<R> primitive(const R q[4], R gm1) {
+__device__ __forceinline__ Prim<R> primitive(const R q[4], R gm1, R inv_rho) {
   Prim<R> w;
   w.rho = q[0];
-  w.inv_rho = rcp(q[0]);
+  w.inv_rho = inv_rho;
   w.u = q[1] * w.inv_rho;
   w.v = q[2] * w.inv_rho;
   w.p = gm1 * (q[3] - R(0.5) * (q[1] * w.u + q[2] * w.v));
   return w;
+}
+template <typename R>
+__device__ __forceinline__ Prim<R> primitive(const R q[4], R gm1) {
+  return primitive(q, gm1, rcp(q[0]));
 }
 
 template <typename R>
@@ -162,12 +166,27 @@ __device__ __forceinline__ void roe(const R qm[4], const R qp[4], const Prim<R>&
   const R a_s = rho * dut;
   const R a_p = (dp + rho * c * dun) * i2c2;
   const R delta = R(0.1) * (abs_(un) + c);
-  const R i2d = rcp(R(2) * delta);
-  auto fixed = [&](R lam) {
-    const R mag = abs_(lam);
-    return mag < delta ? (lam * lam + delta * delta) * i2d : mag;
-  };
-  const R l_m = fixed(un - c), l_p = fixed(un + c), l_0 = abs_(un);
+  R l_m, l_p;
+  const R l_0 = abs_(un);
+  if constexpr (sizeof(R) == 8) {
+    // (FP64: the reciprocal only where a wave is within the fix, a transonic
+    // node; it is a tenth of the flux's double-precision operations)
+    l_m = abs_(un - c);
+    l_p = abs_(un + c);
+    if (l_m < delta || l_p < delta) {
+      const R i2d = rcp(R(2) * delta);
+      if (l_m < delta) l_m = (l_m * l_m + delta * delta) * i2d;
+      if (l_p < delta) l_p = (l_p * l_p + delta * delta) * i2d;
+    }
+  } else {
+    const R i2d = rcp(R(2) * delta);
+    auto fixed = [&](R lam) {
+      const R mag = abs_(lam);
+      return mag < delta ? (lam * lam + delta * delta) * i2d : mag;
+    };
+    l_m = fixed(un - c);
+    l_p = fixed(un + c);
+  }
   const R wmn = l_m * a_m, we = l_0 * a_e, ws = l_0 * a_s, wpl = l_p * a_p;
   const R d0 = wmn + we + wpl;
   const R d1 = wmn * (u - c * nx) + we * u + ws * (-ny) + wpl * (u + c * nx);
@@ -220,16 +239,20 @@ __device__ __forceinline__ void hllc(const R qm[4], const R qp[4], const Prim<R>
 
 // Interface flux Fhat(q-, q+, n) and the normal flux F(q-).n of the interior trace.
 template <typename R, int FLUX>
-__device__ __forceinline__ void interface_flux(const R qm[4], const R qp[4], R nx, R ny, R gamma, R fhat[4], R fm[4]) {
-  const R gm1 = gamma - R(1);
-  const Prim<R> wm = primitive(qm, gm1);
-  const Prim<R> wp = primitive(qp, gm1);
+__device__ __forceinline__ void interface_flux(const R qm[4], const R qp[4], const Prim<R>& wm, R nx, R ny, R gamma,
+                                               R fhat[4], R fm[4]) {
+  const Prim<R> wp = primitive(qp, gamma - R(1));
   R fp[4];
   normal_flux(qm, wm, nx, ny, fm);
   normal_flux(qp, wp, nx, ny, fp);
   if (FLUX == FLUX_RUSANOV) rusanov(qm, qp, wm, wp, nx, ny, gamma, fm, fp, fhat);
   else if (FLUX == FLUX_ROE) roe(qm, qp, wm, wp, nx, ny, gamma, fm, fp, fhat);
   else hllc(qm, qp, wm, wp, nx, ny, gamma, fm, fp, fhat);
+}
+
+template <typename R, int FLUX>
+__device__ __forceinline__ void interface_flux(const R qm[4], const R qp[4], R nx, R ny, R gamma, R fhat[4], R fm[4]) {
+  interface_flux<R, FLUX>(qm, qp, primitive(qm, gamma - R(1)), nx, ny, gamma, fhat, fm);
 }
 
 // Interface flux of a face node as the stage kernels use it. The FP32-mixed

@@ -131,11 +131,6 @@ __global__ void __launch_bounds__(NODE_BS) stage_node_kernel(const StageParams P
     if (MODE != MODE_RHS && !active) live = false;  // a finished instance (uniform in the block)
     if (live) {
       const R gamma = (R)P.gamma, gm1 = gamma - R(1);
-      if (MODE == MODE_LIMITED && P.tape_src && node_lane) {  // adjoint tape: the stage input
-        R* __restrict__ ts = (R*)P.tape_src;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) ts[(size_t)(c * NP + i) * ld + e] = q[c];
-      }
       // ---- contravariant fluxes of the own node
       {
         const Prim<R> w = primitive(q, gm1);
@@ -288,11 +283,6 @@ __global__ void __launch_bounds__(NODE_BS) stage_node_kernel(const StageParams P
         if (node_lane) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) dst[(size_t)(c * NP + i) * ld + e] = acc[c];
-          if (MODE == MODE_LIMITED && P.tape_dst) {  // adjoint tape: the stage result before limiting
-            R* __restrict__ td = (R*)P.tape_dst;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) td[(size_t)(c * NP + i) * ld + e] = acc[c];
-          }
         }
         rmin = fmin(INFINITY, rmin);
         pmin = fmin(INFINITY, pmin);
