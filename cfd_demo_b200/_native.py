@@ -89,6 +89,7 @@ _PROTOS = {
     "cfd_rk3_stage": (C.c_int, [_SP, _p, _p, _p, _i32, _p]),
     "cfd_rk3_finish": (C.c_int, [_SP, _p]),
     "cfd_run_control": (C.c_int, [_SP, _p]),
+    "cfd_rk3_advance": (C.c_int, [_SP, _p, _p, _p, _i32, _p]),
     "cfd_run_init": (C.c_int, [_SP, _p, _p, _p]),
     "cfd_batch_advance": (C.c_int, [_SP, _p, _p, _p, _i32, _p]),
     "cfd_rk3_step_noalloc": (C.c_int, [C.POINTER(CfdMesh), _i32, _i32, _i32, _f64, _f64, _p, _p, _f64, _p, _p]),

@@ -13,7 +13,7 @@ attempts is ONE cooperative launch (cfd_batch_advance) whose blocks stay
 resident, loop over the tiles of every instance and step through the phases
 of each attempt with grid-wide barriers; the chunk's launch is captured in a
 CUDA graph and replayed. ``persistent=False``: CUDA-graph chunks of the
-separate launches (cfd_rk3_attempt + cfd_run_control per attempt). Either
+separate launches (cfd_rk3_advance, six to seven per attempt). Either
 way the host polls the loop states once per chunk. With ``compact=True``,
 once the instances still running hold at most half of the batch's elements,
 `run` / `run_to` repack them into a smaller batch (same tables, states and
@@ -256,12 +256,6 @@ class BatchedEulerSolver:
         _native.check(self._lib.cfd_run_init(C.byref(self._struct), ws.x0.data_ptr(), ftd.data_ptr(), _stream()))
         torch.cuda.current_stream().synchronize()
 
-    def _attempt_and_control(self, stream) -> None:
-        ws = self._ws
-        _native.check(self._lib.cfd_rk3_attempt(C.byref(self._struct), ws.x0.data_ptr(), ws.x1.data_ptr(),
-                                                ws.stage.data_ptr(), stream))
-        _native.check(self._lib.cfd_run_control(C.byref(self._struct), stream))
-
     def _persistent_chunk(self, attempts: int, stream) -> None:
         ws = self._ws
         _native.check(self._lib.cfd_batch_advance(C.byref(self._struct), ws.x0.data_ptr(), ws.x1.data_ptr(),
@@ -271,8 +265,9 @@ class BatchedEulerSolver:
         if self.persistent:
             self._persistent_chunk(n, stream)
         else:
-            for _ in range(n):
-                self._attempt_and_control(stream)
+            ws = self._ws
+            _native.check(self._lib.cfd_rk3_advance(C.byref(self._struct), ws.x0.data_ptr(), ws.x1.data_ptr(),
+                                                    ws.stage.data_ptr(), int(n), stream))
 
     def _chunk_graph(self, n: int):
         import torch

@@ -133,6 +133,18 @@ __global__ void run_init_kernel(CfdControl* ctl, const CfdStageAcc* acc, const d
   ctl[i] = c;
 }
 
+// The end of an attempt of the run loop in one launch: StepReport, control, and
+// (reset) the reduction slots zeroed for the next attempt.
+__global__ void attempt_end_kernel(CfdStageAcc* acc, CfdControl* ctl, CfdStepReport* rep, int n, double cfl,
+                                   int max_rejections, int reset) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  report_one(acc, ctl, rep, i, cfl);
+  control_one(ctl, rep, i, max_rejections);
+  if (reset)
+    for (int k = 0; k < 3; ++k) reset_acc_one(acc, 3 * i + k);
+}
+
 // Loop state of a fixed-size step (cfd_rk3_step_fixed): every instance
 // active, its state in x0, the step size given per instance.
 __global__ void fixed_control_kernel(CfdControl* ctl, const double* dt, int n) {
@@ -567,6 +579,23 @@ int cfd_run_control(const CfdSolver* s, void* stream) {
   const int n = s->mesh.num_instances;
   run_control_kernel<<<blocks_for(n, 128), 128, 0, (cudaStream_t)stream>>>(s->control, s->report, n, s->max_rejections);
   return check_launch("cfd_run_control");
+}
+
+int cfd_rk3_advance(const CfdSolver* s, void* x0, void* x1, void* stage, int32_t attempts, void* stream) {
+  NvtxRange nvtx_range("cfd_rk3_advance");
+  int rc = attempt_args(s, x0, x1, stage);
+  if (rc) return rc;
+  if (attempts < 0) return fail(CFD_E_ARG, "cfd_rk3_advance: attempts must be nonnegative");
+  if (attempts == 0) return CFD_OK;
+  if ((rc = cfd_rk3_begin(s, stream))) return rc;
+  const int n = s->mesh.num_instances;
+  for (int it = 0; it < attempts; ++it) {
+    for (int k = 1; k <= 3; ++k)
+      if ((rc = cfd_rk3_stage(s, x0, x1, stage, k, stream))) return rc;
+    attempt_end_kernel<<<blocks_for(n, 128), 128, 0, (cudaStream_t)stream>>>(s->acc, s->control, s->report, n, s->cfl,
+                                                                             s->max_rejections, it + 1 < attempts);
+  }
+  return check_launch("cfd_rk3_advance");
 }
 
 int cfd_batch_advance(const CfdSolver* s, void* x0, void* x1, void* stage, int32_t attempts, void* stream) {

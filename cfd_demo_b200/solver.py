@@ -9,7 +9,7 @@ shape); outputs are NumPy arrays, as in the reference.
 ``run`` keeps the reference's loop semantics exactly (CFL dt, shortened last
 step, reject-and-halve up to max_rejections, RK-weighted boundary-flux
 accumulation, minima, troubled-cell maximum) but executes the loop body on
-the device (cfd_run_control), so the host only polls the loop state once per
+the device (cfd_rk3_advance), so the host only polls the loop state once per
 chunk of attempts, and each chunk is replayed from a CUDA graph.
 """
 
@@ -389,11 +389,10 @@ class EulerSolver:
         return ws.small[:4].cpu().numpy().copy()
 
     # ---- run loop (solver.py:167-216) ---------------------------------------------
-    def _attempt_and_control(self, stream) -> None:
+    def _issue(self, n: int, stream) -> None:
         ws = self._ws
-        _native.check(self._lib.cfd_rk3_attempt(C.byref(self._struct), ws.x0.data_ptr(), ws.x1.data_ptr(),
-                                                ws.stage.data_ptr(), stream))
-        _native.check(self._lib.cfd_run_control(C.byref(self._struct), stream))
+        _native.check(self._lib.cfd_rk3_advance(C.byref(self._struct), ws.x0.data_ptr(), ws.x1.data_ptr(),
+                                                ws.stage.data_ptr(), int(n), stream))
 
     def _chunk_graph(self, n: int):
         import torch
@@ -404,9 +403,7 @@ class EulerSolver:
             side.wait_stream(torch.cuda.current_stream())
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=side):
-                s = torch.cuda.current_stream().cuda_stream
-                for _ in range(n):
-                    self._attempt_and_control(s)
+                self._issue(n, torch.cuda.current_stream().cuda_stream)
             torch.cuda.current_stream().wait_stream(side)
             self._graphs[n] = g
         return g
@@ -432,9 +429,7 @@ class EulerSolver:
         if graph:
             self._chunk_graph(attempts).replay()
         else:
-            s = _stream()
-            for _ in range(attempts):
-                self._attempt_and_control(s)
+            self._issue(attempts, _stream())
         return self._read(self._ws.control, _native.CfdControl)
 
     def state_tensor(self):

@@ -290,6 +290,11 @@ int cfd_rk3_finish(const CfdSolver* s, void* stream);
  */
 int cfd_run_control(const CfdSolver* s, void* stream);
 
+/* cfd_rk3_advance: `attempts` passes of (cfd_rk3_attempt + cfd_run_control) in
+ * fewer launches: report, control and the next attempt's zeroing are one. The
+ * same results; the reduction slots hold the last attempt's values afterwards. */
+int cfd_rk3_advance(const CfdSolver* s, void* x0, void* x1, void* stage, int32_t attempts, void* stream);
+
 /*
  * cfd_batch_advance: `attempts` passes of (cfd_rk3_attempt + cfd_run_control)
  * for every instance in ONE persistent, cooperative launch (no counterpart in
