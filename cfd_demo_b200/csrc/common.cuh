@@ -376,32 +376,6 @@ __device__ __forceinline__ double pressure_theta(const double a[4], double d0, d
   return lo;
 }
 
-// Nodal minima (density, pressure; NaN ignored), max wave speed and finiteness.
-template <typename R>
-__device__ __forceinline__ void element_stats(const R (&q)[NP][4], double gm1, double gamma, double& rmin, double& pmin,
-                                              double& lam, bool& finite) {
-  rmin = INFINITY;
-  pmin = INFINITY;
-  lam = -INFINITY;
-  finite = true;
-  bool lam_nan = false;
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    const double r = q[i][0], mx = q[i][1], my = q[i][2], en = q[i][3];
-    const double p = node_pressure<R>(q[i][0], q[i][1], q[i][2], q[i][3], gm1, POSITIVITY_FLOOR);
-    rmin = fmin(rmin, r);
-    pmin = fmin(pmin, p);
-    // time_integration.py:39-40: |u| + c
-    const double s = wave_speed<R>(q[i][0], q[i][1], q[i][2], q[i][3], gamma);
-    lam_nan |= (s != s);
-    lam = fmax(lam, s);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) finite &= finite_(q[i][c]);
-  }
-  if (lam_nan) lam = NAN;
-}
-
-
 // One face node of the surface term: exterior state, interface flux, lifted
 // jump, boundary-flux contribution (dg.py:153-164, boundary: dg.py:119-137).
 template <typename R, int FLUX>

@@ -300,7 +300,7 @@ __device__ __forceinline__ void limit_half_warp(const LimitParams& P, int e, int
 #pragma unroll
     for (int k = 0; k < 4; ++k) q[(k * NP + t) * ld + e] = v[k];
   }
-  // ---- statistics of the own node (element_stats in common.cuh); the wave
+  // ---- statistics of the own node; the wave
   // speed only where the CFL step is formed. The minima of the element are left
   // to the block's reduction: dt_geo / speed is monotone, so its least value
   // over the nodes is that of the largest speed.
