@@ -529,13 +529,16 @@ void launch_quad(const StageParams& p, cudaStream_t st) {
 //   2,000    FP64 / FP32            48 /  41             -         107 /  62     112 /  61
 //   8,000    FP64 / FP32           102 /  70            98         105 /  71     105 /  67
 //   32,000   FP64 / FP32           330 / 160           167         213 / 106     237 / 101
-//   1.05 M   FP32                                                  1,432         1,290
+//   65,522   FP32                                                    112           111
+//   125,000  FP32                                                    210           193
+//   1.05 M   FP32                                                  1,428         1,286
 // In FP32-mixed the node form rounds as tiles of 32 do (but for a few sums in
-// the limited stages); tiles of 64 with the flux as a call round more of them
-// differently, which a run near the limiter's thresholds shows, so that choice
-// is left to the autotuner. A batch (flags bit 0) keeps one FP64 kernel at every
-// size, because it may be repacked into a smaller one.
-constexpr int NODE_MAX = 8000;
+// the limited stages); tiles of 64 with the flux as a call (shape 9) round more of
+// them differently, which a run near the slope limiter's thresholds shows: they
+// are taken from TILE64_MIN on where the limiter is `unlimited`, and left to the
+// autotuner otherwise. A batch (flags bit 0) keeps one kernel at every size where
+// two would round differently, because it may be repacked into a smaller one.
+constexpr int NODE_MAX = 8000, TILE64_MIN = 100000;
 // The differentiable step's shape behind variant 0, at every size: tiles of 32.
 // Its gradient takes the branch of |u.n| and of the limiter that round-off picks
 // where a region is uniform, so a kernel that rounds differently would change
@@ -547,6 +550,8 @@ void launch_stage_default(const StageParams& p, cudaStream_t st) {
   if (p.m.ld % 64 || (n <= NODE_MAX && !(sizeof(R) == 8 && (p.m.flags & 1))))
     stage_node_kernel<R, FLUX, MODE><<<blocks_for(n, NODE_EPB), NODE_BS, 0, st>>>(p);
   else if constexpr (sizeof(R) == 8) launch_quad<FLUX, MODE>(p, st);
+  else if (MODE == MODE_UNLIMITED && n >= TILE64_MIN && !(p.m.flags & 1))
+    launch_tile<R, FLUX, MODE, 64, true, 4, true, true, true>(p, st);
   else launch_tile<R, FLUX, MODE, 32, false>(p, st);
 }
 template <typename R, int FLUX, int MODE>

@@ -2,21 +2,16 @@
 // path (the operator of CFD-demo's src/cfd_demo/dg.py, limiting.py and
 // time_integration.py, driven by the run loop of solver.py).
 //
-// Design: one thread per element, element-major SoA state q[(c*15+j)*ld+e], so
-// every per-node load and store of a warp is one coalesced 256 B (double) or
-// 128 B (float) transaction. The 15x30 [Dr|Ds] contraction and the 15x15 LIFT
-// are compile-time constants (tables.cuh) applied as register-blocked FMAs:
-// each thread streams over the nodes j computing the contravariant fluxes
-// once and accumulating into a 15x4 register tile, then streams over its 15
-// face nodes (neighbour trace gathered from the neighbour's column, or a
-// boundary state), evaluates the interface flux and lifts the jump into the
-// same tile. The RK stage combine, the cell averages and — when the limiter
+// Design: element-major SoA state q[(c*15+j)*ld+e], so that a warp's loads of one
+// row are contiguous. A stage is one kernel: the [Dr|Ds] contraction, the face
+// fluxes and LIFT, the RK stage combine, the cell averages and — when the limiter
 // is `unlimited` — the positivity limiter, the stage minima and the CFL
-// reduction all happen in the same kernel, so one stage reads the state once
-// and writes it once. With slope limiting, a second light kernel per stage
-// (limit_kernel) reads the averages of the element and its neighbours plus
-// six midpoint traces and rewrites only troubled or non-positive elements.
-// Global reductions go through ordered 64-bit keys and one atomic per block.
+// reduction; how its work is dealt out (by node, by variable, by element pair)
+// goes by the size of the mesh (launch_stage_default in common.cuh). With slope
+// limiting a second kernel per stage (limit_kernel) reads the averages of the
+// element and its neighbours plus six midpoint traces and rewrites only troubled
+// or non-positive elements. Global reductions go through ordered 64-bit keys and
+// one atomic per block.
 #include "common.cuh"
 
 #include <nvtx3/nvToolsExt.h>
@@ -69,37 +64,50 @@ __global__ void __launch_bounds__(BS) prep_kernel(CfdMesh m, const R* __restrict
 // speed is monotone, so its least value over the nodes is that of the element's
 // largest speed. What bounds it is the divisions and square roots of the wave
 // speed (440 cycles in double, in the reference's order): one thread an element
-// took its 15 nodes in turn, 19 us for 2,000 elements, 256 us for 800,000.
-constexpr int DT_EPB = 32;
+// took its 15 nodes in turn, 19 us for 2,000 elements, 256 us for 800,000. One
+// mesh is swept by as many blocks as are resident, with one commit each (a commit
+// per 32 elements cost 240 us at 1.05 M elements in FP32-mixed).
+constexpr int DT_EPB = 32, DT_BLOCKS = 148 * 4;
 template <typename R>
 __global__ void __launch_bounds__(DT_EPB * NP) dt_kernel(CfdMesh m, const R* __restrict__ q, CfdStageAcc* acc, double gamma) {
-  const int e0 = blockIdx.x * DT_EPB, e = e0 + (threadIdx.x & 31), i = threadIdx.x >> 5;
-  int inst = 0;
-  bool live = e < m.num_elements;
-  bool uniform = true;
-  if (m.instance) {  // (instances start at multiples of 64, or the block's elements commit one by one)
-    inst = live ? m.instance[e] : -1;
-    live = inst >= 0;
-    uniform = __syncthreads_and(!live || inst == m.instance[e0]);
-  }
+  const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
   Red red;
   red.init();
-  if (live) {
+  double rm = INFINITY, pm = INFINITY, dm = INFINITY;
+  auto node = [&](int e) {
     R v[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) v[c] = q[(size_t)(c * NP + i) * m.ld + e];
-    const double d = m.dt_geo[e] / wave_speed<R>(v[0], v[1], v[2], v[3], gamma);
-    red.kd = dkey(d);
-    // time_integration.py:41 — the min propagates NaN: a NaN node poisons dt
-    if (d != d) red.fl |= FLAG_NAN_DT;
-    red.kr = dkey(fmin(INFINITY, (double)v[0]));
-    red.kp = dkey(fmin(INFINITY, node_pressure<R>(v[0], v[1], v[2], v[3], gamma - 1.0, POSITIVITY_FLOOR)));
+    const double speed = wave_speed<R>(v[0], v[1], v[2], v[3], gamma), g = m.dt_geo[e];
+    // the division only where it can lower the least step so far (or is NaN)
+    if (!(g > dm * speed * (1.0 + 1e-12))) {
+      const double d = g / speed;
+      // time_integration.py:41 — the min propagates NaN: a NaN node poisons dt
+      if (d != d) red.fl |= FLAG_NAN_DT;
+      dm = fmin(dm, d);
+    }
+    rm = fmin(rm, (double)v[0]);
+    pm = fmin(pm, node_pressure<R>(v[0], v[1], v[2], v[3], gamma - 1.0, POSITIVITY_FLOOR));
     if (!(finite_(v[0]) && finite_(v[1]) && finite_(v[2]) && finite_(v[3]))) red.fl |= FLAG_NONFINITE;
+  };
+  auto keys = [&]() { red.kr = dkey(rm), red.kp = dkey(pm), red.kd = dkey(dm); };
+  if (!m.instance) {
+    for (int e = blockIdx.x * DT_EPB + lane; e < m.num_elements; e += gridDim.x * DT_EPB) node(e);
+    keys();
+    commit_keys(red, acc + 2);
+    return;
   }
-  if (uniform) {
-    const int first = m.instance ? m.instance[e0] : 0;
+  // several instances, one group of elements per block: they start at multiples
+  // of 64, or the block's elements commit one by one
+  const int e0 = blockIdx.x * DT_EPB, e = e0 + lane;
+  const int inst = e < m.num_elements ? m.instance[e] : -1, first = m.instance[e0];
+  if (inst >= 0) {
+    node(e);
+    keys();
+  }
+  if (__syncthreads_and(inst < 0 || inst == first)) {
     if (first >= 0) commit_keys(red, acc + 3 * first + 2);
-  } else if (live) {
+  } else if (inst >= 0) {
     commit_one(red, acc + 3 * inst + 2);
   }
 }
@@ -363,7 +371,9 @@ static void launch_limit(const CfdSolver* s, const LimitParams& p, cudaStream_t 
 }
 template <typename R>
 static void launch_dt(const CfdSolver* s, const void* q, cudaStream_t st) {
-  dt_kernel<R><<<blocks_for(s->mesh.num_elements, DT_EPB), DT_EPB * NP, 0, st>>>(s->mesh, (const R*)q, s->acc, s->gamma);
+  const unsigned g = blocks_for(s->mesh.num_elements, DT_EPB);
+  dt_kernel<R><<<!s->mesh.instance && g > DT_BLOCKS ? DT_BLOCKS : g, DT_EPB * NP, 0, st>>>(s->mesh, (const R*)q, s->acc,
+                                                                                       s->gamma);
 }
 static void reset_acc(const CfdSolver* s, cudaStream_t st) {
   const int n = 3 * s->mesh.num_instances;
