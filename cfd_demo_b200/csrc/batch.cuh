@@ -35,6 +35,7 @@ template <> struct BatchShape<double> {
   static constexpr int EPB = 64, MINB = 3;
   static constexpr bool SB = false, UF = true, PK = false, CF = false;
 };
+static_assert(BatchShape<float>::EPB == BatchShape<double>::EPB, "cfd_batch_advance checks one tile size");
 
 template <typename R, int FLUX, int PHI>
 __global__ void __launch_bounds__(2 * BatchShape<R>::EPB, BatchShape<R>::MINB)

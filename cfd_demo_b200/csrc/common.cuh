@@ -423,7 +423,7 @@ struct StageParams {
   const void* q_in;  // MODE_RHS
   void* q_out;       // MODE_RHS
   double* bflux_out; // MODE_RHS, [instances][4]
-  void* tape_src;    // optional: copy of the stage input written here (tiled kernels)
+  void* tape_src;    // optional: copy of the stage input written here (tiled kernels only)
   void* tape_dst;    // optional: second copy of the stage result (before limiting)
 };
 
@@ -473,6 +473,11 @@ inline unsigned blocks_for(long long n, int bs) { return (unsigned)((n + bs - 1)
 int cfd_fail(int code, const char* msg);
 
 // ---------------------------------------------------- stage-kernel launches ---
+// The differentiable step's shape behind variant 0, at every size: tiles of 32.
+// Its gradient takes the branch of |u.n| and of the limiter that round-off picks
+// where a region is uniform, so a kernel that rounds differently would change
+// the gradient there (1.9e-4 of its norm on a shock tube), not its last bits.
+constexpr int SHAPE_TILE32 = -1;
 template <typename R, int FLUX, int MODE>
 void launch_stage_bs(const StageParams& p, int bs, cudaStream_t st) {
   const unsigned g = blocks_for(p.m.num_elements, bs / 2);  // two threads per element
@@ -480,11 +485,27 @@ void launch_stage_bs(const StageParams& p, int bs, cudaStream_t st) {
   else if (bs == 256) stage_pair_kernel<R, FLUX, MODE, 256><<<g, 256, 0, st>>>(p);
   else stage_pair_kernel<R, FLUX, MODE, 128><<<g, 128, 0, st>>>(p);
 }
-template <typename R, int MODE>
-void launch_stage_flux(const StageParams& p, int flux, int bs, cudaStream_t st) {
-  if (flux == 0) launch_stage_bs<R, 0, MODE>(p, bs, st);
-  else if (flux == 1) launch_stage_bs<R, 1, MODE>(p, bs, st);
-  else launch_stage_bs<R, 2, MODE>(p, bs, st);
+// Whether a form that copies epb elements of every row by 16 bytes at a time may
+// serve these buffers: the last block's columns end inside the leading dimension,
+// and every row starts at a multiple of 16 bytes (ld a multiple of 4, for the
+// int and float rows). Any ld >= num_elements is a valid mesh; the pair and node
+// forms read element by element and take all of them.
+inline bool staged_fits(const StageParams& p, int precision, int epb) {
+  const CfdMesh& m = p.m;
+  const bool f64 = precision == CFD_FP64;
+  const void* rows[] = {p.q_in, p.x0, p.x1, p.stage, m.face_info, m.neighbor,
+                        f64 ? (const void*)m.metric : (const void*)m.metric32,
+                        f64 ? (const void*)m.face_geo : (const void*)m.face_geo32};
+  for (const void* r : rows)
+    if ((uintptr_t)r % 16) return false;
+  return m.ld % 4 == 0 && ((long long)m.num_elements + epb - 1) / epb * epb <= m.ld;
+}
+// The shape that serves a call asking for `variant`: the pair kernel in place of
+// a tiled shape that does not fit. (Variant 0 is settled in launch_stage_default.)
+inline int staged_variant(const StageParams& p, int precision, int variant) {
+  if (variant == 0 || variant == 2) return variant;
+  const int epb = variant == 1 || variant == 4 || variant == SHAPE_TILE32 ? 32 : 64;
+  return staged_fits(p, precision, epb) ? variant : 2;
 }
 template <typename R, int FLUX, int MODE, int EPB, bool SB, int MINB = (sizeof(R) == 4 ? 512 : 384) / (2 * EPB),
           bool UF = true, bool PK = true, bool CF = false, bool FJ = false, bool VR = false>
@@ -520,9 +541,8 @@ void launch_quad(const StageParams& p, cudaStream_t st) {
   }
   stage_quad_kernel<FLUX, MODE><<<blocks_for(p.m.num_elements, QUAD_EPB), QUAD_BS, BYTES, st>>>(p);
 }
-// Variant 0, by size. One thread per node up to NODE_MAX elements, and on meshes
-// whose leading dimension does not keep the other forms' 16-byte copies aligned
-// and inside a row; above, four lanes per element in FP64 and tiles of 32
+// Variant 0, by size. One thread per node up to NODE_MAX elements, and where the
+// other forms' 16-byte copies do not fit the buffers (staged_fits); above, four lanes per element in FP64 and tiles of 32
 // elements in FP32-mixed. One RK3 attempt (graph replay), us (larger meshes:
 // stage_quad.cuh):
 //   elements                  one thread per node   four lanes   tiles of 32   tiles of 64
@@ -539,21 +559,17 @@ void launch_quad(const StageParams& p, cudaStream_t st) {
 // autotuner otherwise. A batch (flags bit 0) keeps one kernel at every size where
 // two would round differently, because it may be repacked into a smaller one.
 constexpr int NODE_MAX = 8000, TILE64_MIN = 100000;
-// The differentiable step's shape behind variant 0, at every size: tiles of 32.
-// Its gradient takes the branch of |u.n| and of the limiter that round-off picks
-// where a region is uniform, so a kernel that rounds differently would change
-// the gradient there (1.9e-4 of its norm on a shock tube), not its last bits.
-constexpr int SHAPE_TILE32 = -1;
 template <typename R, int FLUX, int MODE>
 void launch_stage_default(const StageParams& p, cudaStream_t st) {
-  const int n = p.m.num_elements;
-  if (p.m.ld % 64 || (n <= NODE_MAX && !(sizeof(R) == 8 && (p.m.flags & 1))))
+  const int n = p.m.num_elements, precision = sizeof(R) == 8 ? CFD_FP64 : CFD_FP32_MIXED;
+  if ((n <= NODE_MAX && !(sizeof(R) == 8 && (p.m.flags & 1))) || !staged_fits(p, precision, 32))
     stage_node_kernel<R, FLUX, MODE><<<blocks_for(n, NODE_EPB), NODE_BS, 0, st>>>(p);
   else if constexpr (sizeof(R) == 8) launch_quad<FLUX, MODE>(p, st);
-  else if (MODE == MODE_UNLIMITED && n >= TILE64_MIN && !(p.m.flags & 1))
+  else if (MODE == MODE_UNLIMITED && n >= TILE64_MIN && !(p.m.flags & 1) && staged_fits(p, precision, 64))
     launch_tile<R, FLUX, MODE, 64, true, 4, true, true, true>(p, st);
   else launch_tile<R, FLUX, MODE, 32, false>(p, st);
 }
+static_assert(QUAD_EPB == 32, "launch_stage_default checks the fit of 32 elements a block");
 template <typename R, int FLUX, int MODE>
 void launch_stage_variant(const StageParams& p, int variant, int bs, cudaStream_t st) {
   if (variant == 2) launch_stage_bs<R, FLUX, MODE>(p, bs, st);

@@ -337,7 +337,7 @@ static inline int bs_of(const CfdSolver* s) { return s->block_size ? s->block_si
 
 static void launch_stage(const CfdSolver* s, const StageParams& p, int mode, cudaStream_t st) {
   const int bs = bs_of(s);
-  const int v = s->variant;
+  const int v = staged_variant(p, s->precision, s->variant);
   if (s->precision == CFD_FP64) {
     if (mode == MODE_RHS) launch_stage_part<double, MODE_RHS>(p, s->flux, v, bs, st);
     else if (mode == MODE_LIMITED) launch_stage_part<double, MODE_LIMITED>(p, s->flux, v, bs, st);
@@ -632,6 +632,15 @@ int cfd_batch_advance(const CfdSolver* s, void* x0, void* x1, void* stage, int32
   b.x1 = x1;
   b.stage = stage;
   b.attempts = attempts;
+  StageParams p;
+  memset(&p, 0, sizeof(p));
+  p.m = s->mesh;
+  p.x0 = x0;
+  p.x1 = x1;
+  p.stage = stage;
+  if (!staged_fits(p, s->precision, BatchShape<double>::EPB))
+    return fail(CFD_E_ARG, "cfd_batch_advance: needs ld a multiple of 4 that holds whole tiles of 64 elements, and "
+                           "states and tables at multiples of 16 bytes");
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e;
   if (s->precision == CFD_FP64) {
@@ -778,8 +787,8 @@ int cfd_rk3_step_fixed(const CfdSolver* s, const void* q_in, void* q_out, void* 
   fixed_control_kernel<<<blocks_for(n, 128), 128, 0, st>>>(s->control, dt, n);
   reset_acc(s, st);
   // with a tape, the tiled stage kernel writes its input tile and its result
-  // into the tape as it goes (the register-only pair kernel cannot copy its
-  // input), and the averages / minima / positivity theta land there directly
+  // into the tape as it goes (the register-only pair kernel, which serves
+  // buffers that no tile fits, cannot copy its input), and the averages / minima / positivity theta land there directly
   CfdSolver sv = *s;
   if (sv.variant == 0 || (tape && sv.variant == 2)) sv.variant = SHAPE_TILE32;
   for (int k = 1; k <= 3; ++k) {
@@ -802,6 +811,9 @@ int cfd_rk3_step_fixed(const CfdSolver* s, const void* q_in, void* q_out, void* 
     // the limited path for every limiter: positivity runs in limit_kernel on
     // the stored stage state, so the tape sees the state before limiting
     launch_stage(&sv, p, MODE_LIMITED, st);
+    if (p.tape_src && staged_variant(p, prec, sv.variant) == 2 &&  // the pair kernel: the stage input as one copy
+        cudaMemcpyAsync(p.tape_src, k == 2 ? q_out : stage, state_bytes(ld, prec), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+      return check_launch("cfd_rk3_step_fixed: tape copy");
     LimitParams lp;
     memset(&lp, 0, sizeof(lp));
     lp.m = s->mesh;

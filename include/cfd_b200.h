@@ -99,7 +99,12 @@ extern "C" {
  */
 typedef struct CfdMesh {
     int32_t num_elements;  /* K: elements of all instances */
-    int32_t ld;            /* leading dimension, >= num_elements */
+    int32_t ld;            /* leading dimension, >= num_elements. The fast forms of the stage
+                              kernel copy whole blocks of 32 or 64 elements by 16 bytes: they
+                              serve an ld that is a multiple of 4 and holds num_elements rounded
+                              up to a block (a multiple of 64 always does), with states and
+                              tables at multiples of 16 bytes. Others are served element by
+                              element (cfd_batch_advance refuses them). */
     int32_t num_instances; /* >= 1 */
     int32_t flags;         /* bit 0: every instance starts at a multiple of 64 elements
                               (padding elements have instance -1); required by the tiled
