@@ -20,6 +20,7 @@ RUN_ACTIVE, RUN_DONE, RUN_BAD_DT, RUN_REJECTED = 0, 1, -1, -2
 NOALLOC_MAX_ELEMENTS = 16384  # CFD_NOALLOC_MAX_ELEMENTS of include/cfd_b200.h
 ADJ_HOLD_THETA = 1  # CFD_ADJ_HOLD_THETA
 LIMIT_LIST_HEADER = 16  # CFD_LIMIT_LIST_HEADER
+NODE_MAX_ELEMENTS = 8000  # CFD_NODE_MAX_ELEMENTS
 ABI_VERSION = 2  # CFD_ABI_VERSION
 
 _p = C.c_void_p

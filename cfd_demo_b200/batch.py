@@ -180,8 +180,9 @@ class BatchedEulerSolver:
         carries on from their current states and loop states (read at a chunk
         boundary). The tables are this batch's host tables (not rebuilt); each
         state is copied into the new batch's first buffer and its loop state's
-        parity set to match. Tiles never straddle instances, so every element
-        is computed exactly as it would have been in this batch."""
+        parity set to match. Tiles never straddle instances and the new batch
+        keeps this one's stage kernel, so every element is computed exactly as
+        it would have been in this batch."""
         import torch
 
         sub = BatchedEulerSolver([self.cases[i] for i in keep], self.config, device=self._device,
@@ -189,9 +190,11 @@ class BatchedEulerSolver:
                                  persistent=self.persistent, compact=self.compact,
                                  _parts=[self._parts[i] for i in keep])
         sub._struct.block_size = self._struct.block_size
-        # one instance left is still a batch: variant 0 then keeps the batch's
-        # FP64 kernel, whose results another one may round differently
-        sub._struct.mesh.flags |= 1
+        # one instance left is still a batch, and one that shrinks below the node
+        # form's limit keeps the kernel of larger ones: variant 0 then stays with
+        # this batch's kernel, whose results another one may round differently
+        large = self._struct.mesh.num_elements > _native.NODE_MAX_ELEMENTS
+        sub._struct.mesh.flags |= 1 | (2 if large else self._struct.mesh.flags & 2)
         raw = bytearray()
         for k, i in enumerate(keep):
             c = _native.CfdControl.from_buffer_copy(bytes(ctl[i]))

@@ -556,13 +556,16 @@ void launch_quad(const StageParams& p, cudaStream_t st) {
 // the limited stages); tiles of 64 with the flux as a call (shape 9) round more of
 // them differently, which a run near the slope limiter's thresholds shows: they
 // are taken from TILE64_MIN on where the limiter is `unlimited`, and left to the
-// autotuner otherwise. A batch (flags bit 0) keeps one kernel at every size where
-// two would round differently, because it may be repacked into a smaller one.
-constexpr int NODE_MAX = 8000, TILE64_MIN = 100000;
+// autotuner otherwise. A batch may be repacked into a smaller one and keeps its
+// kernel then, because another would round differently: in FP64 every batch (flags
+// bit 0) takes four lanes, in FP32-mixed a batch repacked from one above NODE_MAX
+// (flags bit 1) stays with tiles of 32.
+constexpr int NODE_MAX = CFD_NODE_MAX_ELEMENTS, TILE64_MIN = 100000;
 template <typename R, int FLUX, int MODE>
 void launch_stage_default(const StageParams& p, cudaStream_t st) {
   const int n = p.m.num_elements, precision = sizeof(R) == 8 ? CFD_FP64 : CFD_FP32_MIXED;
-  if ((n <= NODE_MAX && !(sizeof(R) == 8 && (p.m.flags & 1))) || !staged_fits(p, precision, 32))
+  const bool node = n <= NODE_MAX && !(p.m.flags & (sizeof(R) == 8 ? 3 : 2));
+  if (node || !staged_fits(p, precision, 32))
     stage_node_kernel<R, FLUX, MODE><<<blocks_for(n, NODE_EPB), NODE_BS, 0, st>>>(p);
   else if constexpr (sizeof(R) == 8) launch_quad<FLUX, MODE>(p, st);
   else if (MODE == MODE_UNLIMITED && n >= TILE64_MIN && !(p.m.flags & 1) && staged_fits(p, precision, 64))

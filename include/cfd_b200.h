@@ -70,6 +70,9 @@ extern "C" {
 /* entries of CfdSolver.limit_list ahead of its element list (counters) */
 #define CFD_LIMIT_LIST_HEADER 16
 
+/* meshes up to this many elements take the stage kernel's node form behind variant 0 */
+#define CFD_NODE_MAX_ELEMENTS 8000
+
 /* run status (CfdControl.status) */
 #define CFD_RUN_ACTIVE 0
 #define CFD_RUN_DONE 1
@@ -108,7 +111,10 @@ typedef struct CfdMesh {
     int32_t num_instances; /* >= 1 */
     int32_t flags;         /* bit 0: every instance starts at a multiple of 64 elements
                               (padding elements have instance -1); required by the tiled
-                              stage kernels when num_instances > 1 */
+                              stage kernels when num_instances > 1.
+                              bit 1: variant 0 takes its form for more than
+                              CFD_NODE_MAX_ELEMENTS elements, whatever num_elements (a batch
+                              repacked from a larger one, whose results must stay the same) */
     const double* metric;    /* [4][ld]  rx, ry, sx, sy */
     const double* face_geo;  /* [9][ld]  nx_f, ny_f, Fscale_f (= sJ/J) for f = 0,1,2 */
     const double* face_hlen; /* [3][ld]  half edge length (boundary-flux weights) */
