@@ -26,7 +26,7 @@ __device__ __forceinline__ R shfl_pair(R v) {
 }
 
 // Positivity limiter on one element held in shared memory as s[c*15 + i]
-// (same arithmetic as `positivity`, node by node, no register tile).
+// (the arithmetic of half_warp_positivity, node by node, no register tile).
 template <typename R>
 __device__ __noinline__ void positivity_smem(R* s, const double* a, double gm1) {
   const double pa = pressure_x(a[0], a[1], a[2], a[3], gm1);
@@ -46,7 +46,19 @@ __device__ __noinline__ void positivity_smem(R* s, const double* a, double gm1) 
     const double q0 = s[i], q1 = s[NP + i], q2 = s[2 * NP + i], q3 = s[3 * NP + i];
     if (!(pressure_near(q0, q1, q2, q3, gm1, pt) < pt)) continue;
     const double d0 = xsub(q0, a[0]), d1 = xsub(q1, a[1]), d2 = xsub(q2, a[2]), d3 = xsub(q3, a[3]);
-    const double lo = pressure_theta(a, d0, d1, d2, d3, gm1, pt);
+    // plain halvings: pressure_theta's registers, in a function called from the
+    // middle of the stage kernels' epilogue, cost their hot path spills (12 bytes a
+    // thread with tiles of 32; a 24-step march of 65,522 elements 2,914 -> 2,838 us
+    // and a 12-step one of 1.05 M 16,007 -> 15,756 us without them)
+    double lo = 0.0, hi = 1.0;
+#pragma unroll 1
+    for (int it = 0; it < BISECTION_STEPS; ++it) {
+      const double mid = xmul(0.5, xadd(lo, hi));
+      const bool ok = pressure_x(xadd(a[0], xmul(mid, d0)), xadd(a[1], xmul(mid, d1)), xadd(a[2], xmul(mid, d2)),
+                                 xadd(a[3], xmul(mid, d3)), gm1) >= pt;
+      lo = ok ? mid : lo;
+      hi = ok ? hi : mid;
+    }
     theta = jmin(theta, lo);
   }
   if (theta < 1.0) {
