@@ -60,16 +60,15 @@ __global__ void __launch_bounds__(BS) prep_kernel(CfdMesh m, const R* __restrict
 
 // ---------------------------------------------------------- small kernels ---
 // Nodal minima (density, pressure; NaN ignored), CFL step and finiteness of a
-// state, one thread per node: a warp holds one node of 32 elements. dt_geo /
-// speed is monotone, so its least value over the nodes is that of the element's
-// largest speed. What bounds it is the divisions and square roots of the wave
-// speed (440 cycles in double, in the reference's order): one thread an element
-// took its 15 nodes in turn, 19 us for 2,000 elements, 256 us for 800,000. One
-// mesh is swept by as many blocks as are resident, with one commit each (a commit
-// per 32 elements cost 240 us at 1.05 M elements in FP32-mixed).
-constexpr int DT_EPB = 32, DT_BLOCKS = 148 * 4;
-template <typename R>
-__global__ void __launch_bounds__(DT_EPB * NP) dt_kernel(CfdMesh m, const R* __restrict__ q, CfdStageAcc* acc, double gamma) {
+// state. FP64: one thread per node, a warp holding one node of 32 elements.
+// dt_geo / speed is monotone, so its least value over the nodes is that of the
+// element's largest speed. What bounds it is the divisions and square roots of
+// the wave speed (440 cycles in double, in the reference's order): one thread an
+// element took its 15 nodes in turn, 19 us for 2,000 elements, 256 us for 800,000.
+// One mesh is swept by DT_BLOCKS blocks at most, with one commit each.
+constexpr int DT_EPB = 32, DT_BLOCKS = 148 * 4;  // two rounds of the two blocks an SM holds
+__global__ void __launch_bounds__(DT_EPB * NP) dt_kernel(CfdMesh m, const double* __restrict__ q, CfdStageAcc* acc, double gamma) {
+  using R = double;
   const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
   Red red;
   red.init();
@@ -110,6 +109,49 @@ __global__ void __launch_bounds__(DT_EPB * NP) dt_kernel(CfdMesh m, const R* __r
   } else if (inst >= 0) {
     commit_one(red, acc + 3 * inst + 2);
   }
+}
+
+// The same in FP32-mixed: one thread per element. The wave speed is a handful of
+// single-precision operations there and the pass is bound by its loads, which a
+// thread's 60 independent ones keep in flight: 110 us at 1.05 M elements (252 MB)
+// where one thread per node took 153, 13.0 us at 2,000 where it took 13.4.
+constexpr int DT_BS = 128;
+__global__ void __launch_bounds__(DT_BS) dt_element_kernel(CfdMesh m, const float* __restrict__ q, CfdStageAcc* acc,
+                                                           double gamma) {
+  const int e = blockIdx.x * DT_BS + threadIdx.x;
+  const int inst_raw = (e < m.num_elements && m.instance) ? m.instance[e] : 0;
+  const bool live = e < m.num_elements && inst_raw >= 0;
+  const int inst = live ? inst_raw : 0;
+  Red red;
+  red.init();
+  if (live) {
+    const int ld = m.ld;
+    float s[NP][4];
+#pragma unroll
+    for (int i = 0; i < NP; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s[i][c] = q[(c * NP + i) * ld + e];
+    double rmin = INFINITY, pmin = INFINITY, lam = -INFINITY;
+    bool finite = true, lam_nan = false;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      rmin = fmin(rmin, (double)s[i][0]);
+      pmin = fmin(pmin, node_pressure<float>(s[i][0], s[i][1], s[i][2], s[i][3], gamma - 1.0, POSITIVITY_FLOOR));
+      const double speed = wave_speed<float>(s[i][0], s[i][1], s[i][2], s[i][3], gamma);
+      lam_nan |= speed != speed;
+      lam = fmax(lam, speed);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) finite &= finite_(s[i][c]);
+    }
+    // time_integration.py:41 — the min propagates NaN: a NaN element poisons dt
+    const double d = lam_nan ? (double)NAN : m.dt_geo[e] / lam;
+    red.kd = dkey(d);
+    if (d != d) red.fl |= FLAG_NAN_DT;
+    red.kr = dkey(rmin);
+    red.kp = dkey(pmin);
+    if (!finite) red.fl |= FLAG_NONFINITE;
+  }
+  block_commit<DT_BS>(red, live, inst, acc, 3, 2);
 }
 
 __global__ void reset_acc_kernel(CfdStageAcc* acc, int n) {
@@ -369,11 +411,15 @@ static void launch_limit(const CfdSolver* s, const LimitParams& p, cudaStream_t 
   if (s->precision == CFD_FP64) launch_limit_lim<double>(p, s->limiter, st);
   else launch_limit_lim<float>(p, s->limiter, st);
 }
-template <typename R>
 static void launch_dt(const CfdSolver* s, const void* q, cudaStream_t st) {
-  const unsigned g = blocks_for(s->mesh.num_elements, DT_EPB);
-  dt_kernel<R><<<!s->mesh.instance && g > DT_BLOCKS ? DT_BLOCKS : g, DT_EPB * NP, 0, st>>>(s->mesh, (const R*)q, s->acc,
-                                                                                       s->gamma);
+  const int n = s->mesh.num_elements;
+  if (s->precision == CFD_FP64) {
+    const unsigned g = blocks_for(n, DT_EPB);
+    dt_kernel<<<!s->mesh.instance && g > DT_BLOCKS ? DT_BLOCKS : g, DT_EPB * NP, 0, st>>>(s->mesh, (const double*)q, s->acc,
+                                                                                         s->gamma);
+  } else {
+    dt_element_kernel<<<blocks_for(n, DT_BS), DT_BS, 0, st>>>(s->mesh, (const float*)q, s->acc, s->gamma);
+  }
 }
 static void reset_acc(const CfdSolver* s, cudaStream_t st) {
   const int n = 3 * s->mesh.num_instances;
@@ -472,8 +518,7 @@ int cfd_time_step(const CfdSolver* s, const void* q, double* dt, void* stream) {
   if (!q || !dt || !s->acc) return fail(CFD_E_ARG, "cfd_time_step: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   reset_acc(s, st);
-  if (s->precision == CFD_FP64) launch_dt<double>(s, q, st);
-  else launch_dt<float>(s, q, st);
+  launch_dt(s, q, st);
   const int n = s->mesh.num_instances;
   dt_out_kernel<<<blocks_for(n, 128), 128, 0, st>>>(s->acc, dt, n, s->cfl);
   return check_launch("cfd_time_step");
@@ -485,8 +530,7 @@ int cfd_check_state(const CfdSolver* s, const void* q, double* out, void* stream
   if (!q || !out || !s->acc) return fail(CFD_E_ARG, "cfd_check_state: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   reset_acc(s, st);
-  if (s->precision == CFD_FP64) launch_dt<double>(s, q, st);
-  else launch_dt<float>(s, q, st);
+  launch_dt(s, q, st);
   const int n = s->mesh.num_instances;
   check_out_kernel<<<blocks_for(n, 128), 128, 0, st>>>(s->acc, out, n);
   return check_launch("cfd_check_state");
@@ -665,8 +709,7 @@ int cfd_run_init(const CfdSolver* s, const void* x0, const double* final_time, v
   if (!x0 || !final_time || !s->control || !s->acc) return fail(CFD_E_ARG, "cfd_run_init: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   reset_acc(s, st);
-  if (s->precision == CFD_FP64) launch_dt<double>(s, x0, st);
-  else launch_dt<float>(s, x0, st);
+  launch_dt(s, x0, st);
   const int n = s->mesh.num_instances;
   run_init_kernel<<<blocks_for(n, 128), 128, 0, st>>>(s->control, s->acc, final_time, n, s->cfl);
   return check_launch("cfd_run_init");
