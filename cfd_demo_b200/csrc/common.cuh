@@ -56,7 +56,8 @@ __device__ __forceinline__ bool finite_(float x) { return isfinite(x); }
 constexpr unsigned long long FN_PACK = tab::FACE_NODES_PACKED;
 
 // FP32 form: skip the [Dr|Ds] entries that are round-off zeros of the
-// construction (|D| < 1e-13: 65 of 225 per matrix). The FP64 form keeps all.
+// construction (|D| < 1e-13: 65 of 225 per matrix). The FP64 form keeps all (but
+// for stage_quad.cuh).
 template <typename R> __host__ __device__ constexpr bool keep_entry(double v) {
   return sizeof(R) == 8 ? true : (v > 1e-13 || v < -1e-13);
 }

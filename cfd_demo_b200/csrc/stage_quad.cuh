@@ -18,7 +18,10 @@
 // Shared rows are padded to 8 words past a multiple of 32, which makes the
 // accesses by node and by variable both free of bank conflicts. The values are
 // the tiled kernel's (stage_tile.cuh) but for the round-off zeros of [Dr|Ds]
-// (65 of 225 entries below 1e-13), which are left out.
+// (65 of 225 entries below 1e-13), which a stage leaves out: its result carries a
+// non-finite node itself, and the step is rejected for it. A right-hand side is
+// handed out as it is: there a sum of zero times every flux carries a non-finite
+// one to all rows of its element, as the dense products of the reference do.
 //
 // What bounds it: instruction issue and the latency of double-precision chains
 // (the FP64 pipe is 41 % busy, 51 % of the issue slots, 16 warps an SM). Two
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(QUAD_BS, 4) stage_quad_kernel(const StageParam
     cp_async_wait<1>();
     __syncwarp();
     const R rx = sm.geo[0][s], ry = sm.geo[1][s], sx = sm.geo[2][s], sy = sm.geo[3][s];
-    R acc[NP + 1];
+    R acc[NP + 1], poison = R(0);
 #pragma unroll
     for (int i = 0; i <= NP; ++i) acc[i] = R(0);
     // ---- volume term
@@ -185,6 +188,7 @@ __global__ void __launch_bounds__(QUAD_BS, 4) stage_quad_kernel(const StageParam
         const int jj = 4 * r + l;
         if (jj >= NP) break;
         const R x = sm.f[c][l][s], y = sm.f[4 + c][l][s];
+        if (MODE == MODE_RHS) poison = fma(R(0), x, fma(R(0), y, poison));
 #pragma unroll
         for (int i = 0; i < NP; ++i)
           if (keep_entry<float>(tab::DR[i][jj])) acc[i] = fma(QUAD_COLUMNS.dr[jj][i], x, acc[i]);
@@ -245,7 +249,7 @@ __global__ void __launch_bounds__(QUAD_BS, 4) stage_quad_kernel(const StageParam
     if (MODE == MODE_RHS) {
       if (live) {
 #pragma unroll
-        for (int i = 0; i < NP; ++i) dst[(size_t)(c * NP + i) * ld + e] = acc[i];
+        for (int i = 0; i < NP; ++i) dst[(size_t)(c * NP + i) * ld + e] = acc[i] + poison;
       }
     } else {
       // ---- SSP-RK3 stage combine (time_integration.py:61-66)
