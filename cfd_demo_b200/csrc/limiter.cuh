@@ -387,6 +387,10 @@ constexpr int LIMIT_BS = 128;
 // kernel, us; the channel's elements are nearly all rewritten, the tube's few.
 //                                 two launches   direct   scan of 32   of 64   of 128
 //   tube,     2,000, FP64              136          104        -          -       -
+//   channel,  6,700, FP64 / FP32         -        83/59     116/87        -       -
+//   channel,  8,200, FP64 / FP32         -        98/67     127/91        -       -
+//   tube,     8,200, FP64 / FP32         -       106/72     113/72        -       -
+//   tube,     9,900, FP64 / FP32         -       116/80     110/76        -       -
 //   tube,    32,000, FP32              170           -         97         93      93
 //   channel, 10,000, FP64               -            -        138        173     218
 //   channel, 40,000, FP64              279           -        231        262     321
@@ -394,10 +398,10 @@ constexpr int LIMIT_BS = 128;
 // (two launches: a scan of the whole mesh, then a rewrite of a global list.)
 // A block that rewrites all it scans takes EPB / 8 rounds of some 4,900 cycles,
 // so few elements a block balance better while the blocks fit the GPU at once
-// (seven of them an SM at 72 registers); the direct form adds nothing once its
-// blocks need more than one wave, and on large meshes the fixed work of a block
-// counts instead.
-constexpr int LIMIT_DIRECT_MAX = 5900, LIMIT_SCAN32_MAX = 70000;
+// (seven of them an SM at 72 registers); in an attempt the direct form is never slower
+// while its blocks of eight elements are one wave (8,288), and on large meshes the
+// fixed work of a block counts instead.
+constexpr int LIMIT_DIRECT_MAX = 148 * 7 * (LIMIT_BS / HALF), LIMIT_SCAN32_MAX = 70000;
 template <typename R, int PHI, int EPB>
 __global__ void __launch_bounds__(LIMIT_BS, 7) limit_kernel(const LimitParams P) {
   limit_block_body<R, PHI, LIMIT_BS, EPB>(P, blockIdx.x * EPB);
