@@ -100,15 +100,17 @@ struct Red {
 
 // Appends e to list[] where flag is set, with one atomic per warp on the
 // shared counter (when a large share of the elements is listed, per-thread
-// atomics on one address serialise). All 32 lanes of the warp must call it.
-__device__ __forceinline__ void warp_list_append(int* list, int* count, bool flag, int e) {
+// atomics on one address serialise), never past list[capacity - 1]. All 32 lanes
+// of the warp must call it.
+__device__ __forceinline__ void warp_list_append(int* list, int* count, bool flag, int e, int capacity = 0x7fffffff) {
   const unsigned mask = __ballot_sync(0xffffffffu, flag);
   if (!mask) return;
   const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
   int base = 0;
   if (lane == leader) base = atomicAdd(count, __popc(mask));
   base = __shfl_sync(0xffffffffu, base, leader);
-  if (flag) list[base + __popc(mask & ((1u << lane) - 1u))] = e;
+  const unsigned at = base + __popc(mask & ((1u << lane) - 1u));
+  if (flag && at < (unsigned)capacity) list[at] = e;
 }
 
 __device__ __forceinline__ void commit_one(const Red& r, CfdStageAcc* a) {

@@ -27,11 +27,13 @@ struct NvtxRange {
 
 namespace cfd {
 
-// Averages + per-element minima of q_in, copied to q_out (cfd_limit prologue).
+// Averages + per-element minima of q_in, copied to q_out, and the limiter's counters
+// zeroed (cfd_limit prologue).
 template <typename R, int BS>
 __global__ void __launch_bounds__(BS) prep_kernel(CfdMesh m, const R* __restrict__ qin, R* __restrict__ qout,
-                                                   double* avg, double* aux, double gamma) {
+                                                   double* avg, double* aux, double gamma, int* limit_counters) {
   const int e = blockIdx.x * BS + threadIdx.x;
+  if (e < 2 && limit_counters) limit_counters[e] = 0;
   if (e >= m.num_elements) return;
   const int ld = m.ld;
   R s[NP][4];
@@ -154,8 +156,9 @@ __global__ void __launch_bounds__(DT_BS) dt_element_kernel(CfdMesh m, const floa
   block_commit<DT_BS>(red, live, inst, acc, 3, 2);
 }
 
-__global__ void reset_acc_kernel(CfdStageAcc* acc, int n) {
+__global__ void reset_acc_kernel(CfdStageAcc* acc, int n, int* limit_counters) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 2 && limit_counters) limit_counters[i] = 0;
   if (i < n) reset_acc_one(acc, i);
 }
 
@@ -393,6 +396,13 @@ static void launch_stage(const CfdSolver* s, const StageParams& p, int mode, cud
 template <typename R, int PHI>
 static void launch_limit_phi(const LimitParams& p, cudaStream_t st) {
   const int n = p.m.num_elements;
+  if constexpr (sizeof(R) == 4) {
+    if (p.list) {
+      limit_scan_kernel<R, PHI><<<blocks_for(n, LIMIT_BS), LIMIT_BS, 0, st>>>(p);
+      limit_rewrite_kernel<R, PHI><<<LIMIT_REWRITE_BLOCKS, LIMIT_BS, 0, st>>>(p);
+      return;
+    }
+  }
   if (n <= LIMIT_DIRECT_MAX) limit_kernel<R, PHI, LIMIT_BS / HALF><<<blocks_for(n, LIMIT_BS / HALF), LIMIT_BS, 0, st>>>(p);
   else if (n <= LIMIT_SCAN32_MAX) limit_kernel<R, PHI, 32><<<blocks_for(n, 32), LIMIT_BS, 0, st>>>(p);
   else limit_kernel<R, PHI, LIMIT_BS><<<blocks_for(n, LIMIT_BS), LIMIT_BS, 0, st>>>(p);
@@ -407,7 +417,14 @@ static void launch_limit_lim(const LimitParams& p, int lim, cudaStream_t st) {
     default: launch_limit_phi<R, 4>(p, st); break;
   }
 }
-static void launch_limit(const CfdSolver* s, const LimitParams& p, cudaStream_t st) {
+static bool limit_two_launches(const CfdSolver* s) {
+  return s->limit_list && s->precision == CFD_FP32_MIXED && s->mesh.num_elements > LIMIT_SCAN32_MAX;
+}
+static void launch_limit(const CfdSolver* s, LimitParams p, cudaStream_t st) {
+  if (limit_two_launches(s)) {
+    p.count = s->limit_list;
+    p.list = s->limit_list + CFD_LIMIT_LIST_HEADER;
+  }
   if (s->precision == CFD_FP64) launch_limit_lim<double>(p, s->limiter, st);
   else launch_limit_lim<float>(p, s->limiter, st);
 }
@@ -423,7 +440,7 @@ static void launch_dt(const CfdSolver* s, const void* q, cudaStream_t st) {
 }
 static void reset_acc(const CfdSolver* s, cudaStream_t st) {
   const int n = 3 * s->mesh.num_instances;
-  reset_acc_kernel<<<blocks_for(n, 128), 128, 0, st>>>(s->acc, n);
+  reset_acc_kernel<<<blocks_for(n, 128), 128, 0, st>>>(s->acc, n, limit_two_launches(s) ? s->limit_list : nullptr);
 }
 
 extern "C" {
@@ -493,10 +510,13 @@ int cfd_limit(const CfdSolver* s, const void* q_in, void* q_out, int32_t* troubl
     return check_launch("cfd_limit: memset");
   const int bs = 128;
   const unsigned g = blocks_for(s->mesh.num_elements, bs);
+  int* counters = limit_two_launches(s) ? s->limit_list : nullptr;
   if (s->precision == CFD_FP64)
-    prep_kernel<double, 128><<<g, bs, 0, st>>>(s->mesh, (const double*)q_in, (double*)q_out, s->averages, s->element_aux, s->gamma);
+    prep_kernel<double, 128><<<g, bs, 0, st>>>(s->mesh, (const double*)q_in, (double*)q_out, s->averages, s->element_aux, s->gamma,
+                                              counters);
   else
-    prep_kernel<float, 128><<<g, bs, 0, st>>>(s->mesh, (const float*)q_in, (float*)q_out, s->averages, s->element_aux, s->gamma);
+    prep_kernel<float, 128><<<g, bs, 0, st>>>(s->mesh, (const float*)q_in, (float*)q_out, s->averages, s->element_aux, s->gamma,
+                                              counters);
   LimitParams p;
   memset(&p, 0, sizeof(p));
   p.m = s->mesh;

@@ -1,6 +1,6 @@
 // limiter.cuh — the Cockburn-Shu troubled-cell limiter and the Zhang-Shu
 // positivity limiter of a stage state (limiting.py:136-216 of CFD-demo), as
-// per-element bodies and the kernel that runs them.
+// per-element bodies and the kernels that run them.
 // Included by common.cuh inside namespace cfd.
 #pragma once
 
@@ -19,6 +19,8 @@ struct LimitParams {
   CfdStageAcc* acc;       // stage mode
   int32_t* troubled_out;  // cfd_limit mode
   double* pos_out;        // optional [2][ld]: pressure-scaling theta and its critical node
+  int* list;              // two launches: the elements to rewrite, and
+  int* count;             // [2] their number and a count of blocks, zero before and after the pair
   uint8_t* flags;         // optional [ld]: troubled-cell indicator per element
 };
 
@@ -315,6 +317,23 @@ __device__ __forceinline__ void limit_half_warp(const LimitParams& P, int e, int
   __syncwarp(hmask);  // the half warp's next element reuses sm
 }
 
+// Adds the reductions of an element of instance i to those of its block, whose
+// instance is inst0; an element of another instance (possible where instances are
+// not aligned to blocks) commits by itself.
+__device__ __forceinline__ void limit_take(const LimitParams& P, const Red& r, int i, int inst0, Red& red) {
+  if (i == inst0) red.merge(r);
+  else if (P.stage_idx != 0) commit_one(r, P.acc + 3 * i + (P.stage_idx - 1));
+  else if (r.tr) atomicAdd(&P.troubled_out[i], r.tr);
+}
+__device__ __forceinline__ void limit_commit(const LimitParams& P, const Red& red, int inst0) {
+  if (P.stage_idx == 0) {
+    const int n = __reduce_add_sync(0xffffffffu, red.tr);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&P.troubled_out[inst0], n);
+  } else {
+    commit_keys(red, P.acc + 3 * inst0 + (P.stage_idx - 1));
+  }
+}
+
 // The limiter on the elements e0 .. e0 + EPB - 1 by a block of BS threads.
 //   EPB = BS: every thread scans one element, the block lists those the
 //     limiters change in shared memory, and its BS / 16 half warps rewrite
@@ -322,10 +341,9 @@ __device__ __forceinline__ void limit_half_warp(const LimitParams& P, int e, int
 //     the rewrite needs no other block.
 //   EPB = BS / 16: each half warp takes one element directly, no list (smaller
 //     meshes, where the scan would only lengthen the chain).
-// The block reduces to one commit; an element of another instance than the
-// block's lowest live one (possible where instances are not aligned to blocks)
-// commits by itself.
-template <typename R, int PHI, int BS, int EPB>
+//   GLOBAL (EPB = BS): the scan alone; the listed elements go to P.list, for
+//     limit_rewrite_kernel.
+template <typename R, int PHI, int BS, int EPB, bool GLOBAL = false>
 __device__ __forceinline__ void limit_block_body(const LimitParams& P, const int e0) {
   constexpr bool SCAN = EPB > BS / HALF;
   __shared__ LimitShared<R> s_half[BS / HALF];
@@ -353,33 +371,25 @@ __device__ __forceinline__ void limit_block_body(const LimitParams& P, const int
   red.init();
   own.init();
   if (SCAN) {
-    if (live && limit_scan_one<R, PHI>(P, e, inst, own)) s_list[atomicAdd(&s_count, 1)] = e;
+    const bool listed = live && limit_scan_one<R, PHI>(P, e, inst, own);
+    if (GLOBAL) warp_list_append(P.list, P.count, listed, e, m.num_elements);
+    else if (listed) s_list[atomicAdd(&s_count, 1)] = e;
   } else {
     if (live) limit_half_warp<R, PHI>(P, e, inst, t, hmask, base, sm, false, own);
   }
   __syncthreads();
   const int inst0 = m.instance ? s_inst : 0;
-  auto take = [&](const Red& r, int i) {
-    if (i == inst0) red.merge(r);
-    else if (P.stage_idx != 0) commit_one(r, P.acc + 3 * i + (P.stage_idx - 1));
-    else if (r.tr) atomicAdd(&P.troubled_out[i], r.tr);
-  };
-  if (live) take(own, inst);
-  if (SCAN) {
+  if (live) limit_take(P, own, inst, inst0, red);
+  if (SCAN && !GLOBAL) {
     for (int k = threadIdx.x / HALF; k < s_count; k += BS / HALF) {
       const int le = s_list[k];
       const int li = m.instance ? m.instance[le] : 0;
       own.init();
       limit_half_warp<R, PHI>(P, le, li, t, hmask, base, sm, true, own);
-      take(own, li);
+      limit_take(P, own, li, inst0, red);
     }
   }
-  if (P.stage_idx == 0) {
-    const int n = __reduce_add_sync(0xffffffffu, red.tr);
-    if (lane == 0 && n) atomicAdd(&P.troubled_out[inst0], n);
-  } else if (inst0 != 0x7fffffff) {
-    commit_keys(red, P.acc + 3 * inst0 + (P.stage_idx - 1));
-  }
+  if (inst0 != 0x7fffffff) limit_commit(P, red, inst0);
 }
 
 constexpr int LIMIT_BS = 128;
@@ -395,14 +405,83 @@ constexpr int LIMIT_BS = 128;
 //   channel, 10,000, FP64               -            -        138        173     218
 //   channel, 40,000, FP64              279           -        231        262     321
 //   tube,   800,000, FP64            3,373           -         -          -     3,236
-// (two launches: a scan of the whole mesh, then a rewrite of a global list.)
+// (two launches here: a scan of the whole mesh, then a rewrite of a global list with
+// four lanes an element.)
 // A block that rewrites all it scans takes EPB / 8 rounds of some 4,900 cycles,
 // so few elements a block balance better while the blocks fit the GPU at once
 // (seven of them an SM at 72 registers); in an attempt the direct form is never slower
 // while its blocks of eight elements are one wave (8,288), and on large meshes the
-// fixed work of a block counts instead.
+// fixed work of a block counts instead. There a troubled region is then a long
+// chain in a few blocks, which in FP32-mixed, with its faster stages, made the
+// attempt slower than a rewrite of a global list. FP32-mixed meshes above LIMIT_SCAN32_MAX therefore scan
+// and rewrite in two launches, the listed elements dealt out one by one to the half
+// warps of the grid. One attempt, us (FP32-mixed; channel and waves: many troubled
+// elements side by side, tube: few):
+//                       four lanes, global list   scan of 32   of 64   of 128   two launches
+//   tube,     72,000               219                172        161      155        165
+//   channel,  90,000               231                204        226      272        183
+//   waves,   180,000               482                431        438      470        371
+//   waves,   500,000               942                989        939      976        831
+//   tube,    800,000             1,384              1,463      1,325    1,258      1,259
+// In FP64 the single launch was nowhere slower than the four-lane rewrite (channel,
+// 90,000: 439 against 530) and stays.
 constexpr int LIMIT_DIRECT_MAX = 148 * 7 * (LIMIT_BS / HALF), LIMIT_SCAN32_MAX = 70000;
+constexpr int LIMIT_REWRITE_BLOCKS = 148 * 3;  // 3,552 half warps; seven blocks an SM cost a tube 2 % more
 template <typename R, int PHI, int EPB>
 __global__ void __launch_bounds__(LIMIT_BS, 7) limit_kernel(const LimitParams P) {
   limit_block_body<R, PHI, LIMIT_BS, EPB>(P, blockIdx.x * EPB);
+}
+
+// Least keys and joint flags of a half warp's lanes in each of them.
+__device__ __forceinline__ void half_warp_join(Red& r, unsigned hmask) {
+#pragma unroll
+  for (int o = 1; o < HALF; o <<= 1) {
+    r.kr = min(r.kr, __shfl_xor_sync(hmask, r.kr, o));
+    r.kp = min(r.kp, __shfl_xor_sync(hmask, r.kp, o));
+    r.kd = min(r.kd, __shfl_xor_sync(hmask, r.kd, o));
+  }
+  r.fl = __reduce_or_sync(hmask, (unsigned)r.fl);
+}
+
+// The rewrite of the elements that a GLOBAL scan has listed, dealt out one by one
+// to the half warps of the whole grid. The last block to finish zeroes the counters
+// for the next pair of launches. (Counters that a caller has not zeroed could make
+// it read entries no scan has written: what is no element is left out.)
+template <typename R, int PHI>
+__global__ void __launch_bounds__(LIMIT_BS, 7) limit_rewrite_kernel(const LimitParams P) {
+  constexpr int EPB = LIMIT_BS / HALF;
+  __shared__ LimitShared<R> s_half[EPB];
+  __shared__ int s_n;
+  const CfdMesh& m = P.m;
+  auto element = [&](int k) {
+    const int e = P.list[k];
+    return (unsigned)e < (unsigned)m.num_elements ? e : -1;
+  };
+  if (threadIdx.x == 0) s_n = min(*(volatile int*)P.count, m.num_elements);
+  __syncthreads();
+  const int n = s_n, first = blockIdx.x * EPB;
+  if (first < n) {
+    const int lane = threadIdx.x & 31, t = lane & (HALF - 1), base = lane & HALF;
+    const unsigned hmask = 0xffffu << base;
+    const int e0 = element(first), inst0 = m.instance && e0 >= 0 ? m.instance[e0] : 0;
+    Red red, own;
+    red.init();
+    for (int k = first + (int)threadIdx.x / HALF; k < n; k += gridDim.x * EPB) {
+      const int e = element(k), inst = m.instance && e >= 0 ? m.instance[e] : 0;
+      if (e < 0 || inst < 0) continue;
+      own.init();
+      limit_half_warp<R, PHI>(P, e, inst, t, hmask, base, s_half[threadIdx.x / HALF], true, own);
+      if (inst != inst0 && P.stage_idx != 0) {  // a batch's list mixes instances: one commit an element
+        half_warp_join(own, hmask);
+        if (t != 0) own.init();
+      }
+      limit_take(P, own, inst, inst0, red);
+    }
+    limit_commit(P, red, inst0);
+  }
+  if (threadIdx.x == 0 && atomicAdd(&P.count[1], 1) == (int)gridDim.x - 1) P.count[0] = P.count[1] = 0;
+}
+template <typename R, int PHI>
+__global__ void __launch_bounds__(LIMIT_BS) limit_scan_kernel(const LimitParams P) {
+  limit_block_body<R, PHI, LIMIT_BS, LIMIT_BS, true>(P, blockIdx.x * LIMIT_BS);
 }

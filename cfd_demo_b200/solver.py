@@ -143,7 +143,7 @@ class Workspace:
         self.control = torch.zeros(n * _native.SIZES["CfdControl"], dtype=torch.uint8, device=dev)
         self.small = torch.zeros(max(4 * n, 3 * n, 8), dtype=torch.float64, device=dev)
         self.small_i = torch.zeros(max(n, 8), dtype=torch.int32, device=dev)
-        # scratch the C ABI still accepts (cfd_batch_advance asks for it)
+        # the limiter's counters and element list (large FP32-mixed meshes)
         self.limit_list = torch.zeros(_native.LIMIT_LIST_HEADER + ops.ld, dtype=torch.int32, device=dev)
         # per-stage troubled-cell indicator, written only when recording is on
         self.flags = torch.zeros((3, ops.ld), dtype=torch.uint8, device=dev)

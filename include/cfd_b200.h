@@ -67,7 +67,7 @@ extern "C" {
 #define CFD_FACE_FIXED_STATE 2
 #define CFD_FACE_EXACT_STATE 3
 
-/* entries of CfdSolver.limit_list ahead of its element list (counters) */
+/* entries of CfdSolver.limit_list ahead of its element list (two counters and padding) */
 #define CFD_LIMIT_LIST_HEADER 16
 
 /* meshes up to this many elements take the stage kernel's node form behind variant 0 */
@@ -233,9 +233,12 @@ typedef struct CfdSolver {
                               12 / 13 as 9 with the volume node loop kept rolled ([Dr|Ds] from
                               the constant bank), with unrolled / rolled face rounds,
                               14 as 5 with the volume node loop kept rolled */
-    int32_t* limit_list;   /* optional [CFD_LIMIT_LIST_HEADER + ld] scratch; the limiter lists the
-                              elements it rewrites per block and no longer uses it
-                              (cfd_batch_advance still asks for it) */
+    int32_t* limit_list;   /* optional [CFD_LIMIT_LIST_HEADER + ld] scratch: with it the FP32-mixed
+                              limiter of a mesh above 70,000 elements lists the elements it
+                              rewrites for a launch of their own (else each block rewrites
+                              those it finds; the same results). cfd_rk3_begin and cfd_limit
+                              zero its counters, and the limiter leaves them at zero.
+                              cfd_batch_advance asks for it and does not use it. */
     uint8_t* troubled_flags; /* optional [3][ld]: the troubled-cell indicator of limiting.py:147-151
                               (1 = troubled, 0 = not) of every active element; stage k of an attempt
                               writes row k-1, cfd_limit writes row 0. NULL: not written. */

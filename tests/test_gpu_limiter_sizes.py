@@ -1,5 +1,6 @@
 """The limiter on both sides of every size at which its form changes: a half warp per element up to
-8,288 elements, blocks that scan 32 up to 70,000, above them blocks that scan 128."""
+8,288 elements, blocks that scan 32 up to 70,000, above them blocks that scan 128 (FP64, or without the
+list scratch) and a launch of its own for the listed elements (FP32-mixed with it)."""
 
 from __future__ import annotations
 
@@ -62,3 +63,28 @@ def test_limit_matches_the_oracle_on_both_sides_of_each_size(nx, ny, rough, prec
         same = flags == troubled
         assert same.mean() > 0.9
         assert np.max(np.abs(got - want)[:, same] / scale) <= 2e-5
+
+
+@pytest.mark.parametrize("nx,ny", [(3889, 9), (300, 150)])
+@pytest.mark.parametrize("limiter", ["minmod", "unlimited", "van_leer"])
+@pytest.mark.parametrize("rough", [0.05, 1.0])
+def test_the_launch_for_listed_elements_is_bitwise_the_single_launch(nx, ny, limiter, rough):
+    """FP32-mixed above 70,000 elements with and without the list scratch: limited states, flags, counts
+    and the reports of repeated steps bit for bit (no tolerance: the same operations; the boundary flux
+    sums atomics in any order)."""
+    s = _solver(nx, ny, limiter, "fp32_mixed")
+    q = _state(s, rough)
+    scratch = s.native.limit_list
+    out = []
+    for use in (scratch, None):
+        s.native.limit_list = use
+        limited, flags = s.limit_with_flags(q)
+        dt, x, reports = s.time_step(q), q, []
+        for _ in range(3):
+            x, r = s.step(x, 0.2 * dt)
+            reports.append((r.admissible, r.min_density, r.min_pressure, r.troubled_cells))
+        out.append((limited, flags, x, reports))
+    s.native.limit_list = scratch
+    for a, b in zip(out[0][:3], out[1][:3]):
+        assert np.array_equal(a, b)
+    assert out[0][3] == out[1][3]
