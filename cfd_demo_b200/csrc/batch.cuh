@@ -88,8 +88,16 @@ __global__ void __launch_bounds__(2 * BatchShape<R>::EPB, BatchShape<R>::MINB)
       grid.sync();
       if constexpr (PHI != LIM_UNLIMITED) {
         lp.stage_idx = k;
+        // in the tile's shared memory: 5 KB beside it would cost FP64 its third block an SM
+        // (an attempt of 159,540 elements 1,012 us instead of 850)
+        constexpr int HALVES = LIMIT_BS / HALF;
+        static_assert(HALVES * sizeof(LimitShared<R>) + LIMIT_BS * sizeof(int) <= TileLayout<R, EPB, SH::SB>::BYTES,
+                      "the limiter works in the tile's memory");
+        extern __shared__ __align__(16) unsigned char smem_raw[];
+        LimitShared<R>* s_half = reinterpret_cast<LimitShared<R>*>(smem_raw);
+        int* s_list = reinterpret_cast<int*>(s_half + HALVES);
         for (int e0 = blockIdx.x * LIMIT_BS; e0 < K; e0 += gridDim.x * LIMIT_BS) {
-          limit_block_body<R, PHI, LIMIT_BS, LIMIT_BS>(lp, e0);
+          limit_block_body<R, PHI, LIMIT_BS, LIMIT_BS, false, true>(lp, e0, s_half, s_list);
           __syncthreads();  // the next block of elements reuses the shared list
         }
         grid.sync();

@@ -343,12 +343,16 @@ __device__ __forceinline__ void limit_commit(const LimitParams& P, const Red& re
 //     meshes, where the scan would only lengthen the chain).
 //   GLOBAL (EPB = BS): the scan alone; the listed elements go to P.list, for
 //     limit_rewrite_kernel.
-template <typename R, int PHI, int BS, int EPB, bool GLOBAL = false>
-__device__ __forceinline__ void limit_block_body(const LimitParams& P, const int e0) {
+//   EXTERNAL: the caller lends the shared memory, BS / 16 LimitShared and EPB ints.
+template <typename R, int PHI, int BS, int EPB, bool GLOBAL = false, bool EXTERNAL = false>
+__device__ __forceinline__ void limit_block_body(const LimitParams& P, const int e0, LimitShared<R>* lent_half = nullptr,
+                                                 int* lent_list = nullptr) {
   constexpr bool SCAN = EPB > BS / HALF;
-  __shared__ LimitShared<R> s_half[BS / HALF];
-  __shared__ int s_list[SCAN ? EPB : 1];
+  __shared__ LimitShared<R> own_half[EXTERNAL ? 1 : BS / HALF];
+  __shared__ int own_list[SCAN && !EXTERNAL ? EPB : 1];
   __shared__ int s_count, s_inst;
+  LimitShared<R>* const s_half = EXTERNAL ? lent_half : own_half;
+  int* const s_list = EXTERNAL ? lent_list : own_list;
   const CfdMesh& m = P.m;
   const int lane = threadIdx.x & 31, t = lane & (HALF - 1), base = lane & HALF;
   const unsigned hmask = 0xffffu << base;
