@@ -544,10 +544,10 @@ void launch_quad(const StageParams& p, cudaStream_t st) {
   }
   stage_quad_kernel<FLUX, MODE><<<blocks_for(p.m.num_elements, QUAD_EPB), QUAD_BS, BYTES, st>>>(p);
 }
-// Variant 0, by size. One thread per node up to NODE_MAX elements, and where the
-// other forms' 16-byte copies do not fit the buffers (staged_fits); above, four lanes per element in FP64 and tiles of 32
-// elements in FP32-mixed. One RK3 attempt (graph replay), us (larger meshes:
-// stage_quad.cuh):
+// Variant 0, by size. One thread per node on small meshes, and where the other
+// forms' 16-byte copies do not fit the buffers (staged_fits); above, four lanes per
+// element or tiles of 32 elements in FP64 and tiles of 32 in FP32-mixed. One RK3
+// attempt (graph replay), us (larger meshes: stage_quad.cuh):
 //   elements                  one thread per node   four lanes   tiles of 32   tiles of 64
 //   2,000    FP64 / FP32            48 /  41             -         107 /  62     112 /  61
 //   8,000    FP64 / FP32           102 /  70            98         105 /  71     105 /  67
@@ -555,6 +555,21 @@ void launch_quad(const StageParams& p, cudaStream_t st) {
 //   65,522   FP32                                                    112           111
 //   125,000  FP32                                                    210           193
 //   1.05 M   FP32                                                  1,428         1,286
+// What decides in FP64 is waves of resident blocks. The node form holds 2,368
+// elements a wave (two blocks of 8 an SM): its third wave ends at 7,104, and the
+// fourth makes a stage slower than four lanes (7,938 elements, unlimited, Rusanov /
+// Roe / HLLC: 71 / 73 / 81 us an attempt against 66 / 71 / 72); a bare right-hand
+// side keeps it up to 8,000 (17 / 18 / 21 us a call against 21 / 22 / 23). Four
+// lanes hold 18,944 elements a wave, tiles of 32 hold 23,680 and are the faster
+// blocks with Rusanov and Roe fluxes, the slower ones with HLLC and where the last
+// tile is ragged. Tiles of 32 over four lanes, time of an unlimited attempt / of a
+// right-hand side (of a tube's, Roe, 8,200 and 12,500 elements: 1.12 and 1.16):
+//   elements   divisible by 32      Rusanov        Roe           HLLC
+//   12,000           yes          0.85 / 0.84   0.87 / 0.88   1.05 / 1.01
+//   12,322           no           1.09 / 0.93   1.16 / 0.98   1.41 / 1.17
+//   20,000           yes          0.77 / 0.79   0.80 / 0.82   0.89 / 0.87
+//   20,402           no           0.93 / 0.86   0.98 / 0.95   1.12 / 1.06
+//   24,000           yes          1.16 / 0.99   1.19 / 1.07   1.37 / 1.21
 // In FP32-mixed the node form rounds as tiles of 32 do (but for a few sums in
 // the limited stages); tiles of 64 with the flux as a call (shape 9) round more of
 // them differently, which a run near the slope limiter's thresholds shows: they
@@ -564,14 +579,24 @@ void launch_quad(const StageParams& p, cudaStream_t st) {
 // bit 0) takes four lanes, in FP32-mixed a batch repacked from one above NODE_MAX
 // (flags bit 1) stays with tiles of 32.
 constexpr int NODE_MAX = CFD_NODE_MAX_ELEMENTS, TILE64_MIN = 100000;
+constexpr int NODE_WAVE64 = 148 * 2 * NODE_EPB, QUAD_WAVE = 148 * 4 * QUAD_EPB, TILE32_WAVE64 = 148 * 5 * 32;
+template <int FLUX, int MODE>
+bool tile32_over_quad(int n) {
+  if (n > TILE32_WAVE64) return false;
+  if (FLUX == FLUX_HLLC) return n % 32 == 0 && n > QUAD_WAVE;
+  return n % 32 == 0 || n > QUAD_WAVE || (MODE == MODE_RHS && FLUX == FLUX_RUSANOV);
+}
 template <typename R, int FLUX, int MODE>
 void launch_stage_default(const StageParams& p, cudaStream_t st) {
   const int n = p.m.num_elements, precision = sizeof(R) == 8 ? CFD_FP64 : CFD_FP32_MIXED;
-  const bool node = n <= NODE_MAX && !(p.m.flags & (sizeof(R) == 8 ? 3 : 2));
+  const int node_max = sizeof(R) == 8 && MODE != MODE_RHS ? 3 * NODE_WAVE64 : NODE_MAX;
+  const bool node = n <= node_max && !(p.m.flags & (sizeof(R) == 8 ? 3 : 2));
   if (node || !staged_fits(p, precision, 32))
     stage_node_kernel<R, FLUX, MODE><<<blocks_for(n, NODE_EPB), NODE_BS, 0, st>>>(p);
-  else if constexpr (sizeof(R) == 8) launch_quad<FLUX, MODE>(p, st);
-  else if (MODE == MODE_UNLIMITED && n >= TILE64_MIN && !(p.m.flags & 1) && staged_fits(p, precision, 64))
+  else if constexpr (sizeof(R) == 8) {
+    if (tile32_over_quad<FLUX, MODE>(n) && !(p.m.flags & 3)) launch_tile<R, FLUX, MODE, 32, false>(p, st);
+    else launch_quad<FLUX, MODE>(p, st);
+  } else if (MODE == MODE_UNLIMITED && n >= TILE64_MIN && !(p.m.flags & 1) && staged_fits(p, precision, 64))
     launch_tile<R, FLUX, MODE, 64, true, 4, true, true, true>(p, st);
   else launch_tile<R, FLUX, MODE, 32, false>(p, st);
 }
