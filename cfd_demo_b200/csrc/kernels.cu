@@ -62,15 +62,29 @@ __global__ void __launch_bounds__(BS) prep_kernel(CfdMesh m, const R* __restrict
 
 // ---------------------------------------------------------- small kernels ---
 // Nodal minima (density, pressure; NaN ignored), CFL step and finiteness of a
-// state. FP64: one thread per node, a warp holding one node of 32 elements.
-// dt_geo / speed is monotone, so its least value over the nodes is that of the
-// element's largest speed. What bounds it is the divisions and square roots of
-// the wave speed (440 cycles in double, in the reference's order): one thread an
-// element took its 15 nodes in turn, 19 us for 2,000 elements, 256 us for 800,000.
-// One mesh is swept by DT_BLOCKS blocks at most, with one commit each.
-constexpr int DT_EPB = 32, DT_BLOCKS = 148 * 4;  // two rounds of the two blocks an SM holds
-__global__ void __launch_bounds__(DT_EPB * NP) dt_kernel(CfdMesh m, const double* __restrict__ q, CfdStageAcc* acc, double gamma) {
-  using R = double;
+// state, one thread per node: a warp holds one node of 32 elements. dt_geo / speed
+// is monotone, so its least value over the nodes is that of the element's largest
+// speed. What bounds it in FP64 is the divisions and square roots of the wave speed
+// (440 cycles, in the reference's order): one thread an element took its 15 nodes
+// in turn. It is swept by as many blocks as are resident (two an SM), in one mesh
+// with one commit each. cfd_time_step, us:
+//   elements                         by element   by node   twice as many blocks
+//   2,000               FP64 / FP32   16.9 / 8.5   5.7 / 5.1       5.7 / 5.1
+//   20,000              FP64 / FP32   12.3 / 9.3   8.2 / 7.2       9.4 / 8.4
+//   72,000              FP64 / FP32   32.8 / 9.6  21.5 / 11.1     21.8 / 12.1
+//   160,000             FP64 / FP32   32.5 / 20.5 26.6 / 16.9     28.0 / 18.5
+//   299,000             FP64 / FP32   65.9 / 29.7 59.2 / 30.0     59.1 / 30.9
+//   1.0 M               FP64 / FP32    193 / 101   178 / 135       182 / 139
+//   24 inst., 509,518   FP64 / FP32    164 / 58    167 / 114       169 / 116
+//   16 inst.,  58,702   FP64 / FP32   33.5 / 10.4 23.5 / 14.2     25.8 / 16.0
+//   14 inst.,  13,344   FP64 / FP32   17.8 /  9.9 10.4 /  8.6     10.3 /  9.0
+// FP32-mixed wave speeds are a handful of operations; there the pass is bound by its
+// loads on large meshes, which a thread's 60 independent ones keep in flight, and
+// takes an element a thread from DT_NODE_MAX32 elements on (several instances, whose
+// changes cost commits, from DT_NODE_MAX32_BATCH on).
+constexpr int DT_EPB = 32, DT_BLOCKS = 148 * 2, DT_NODE_MAX32 = 300000, DT_NODE_MAX32_BATCH = 20000;
+template <typename R>
+__global__ void __launch_bounds__(DT_EPB * NP) dt_kernel(CfdMesh m, const R* __restrict__ q, CfdStageAcc* acc, double gamma) {
   const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
   Red red;
   red.init();
@@ -98,25 +112,47 @@ __global__ void __launch_bounds__(DT_EPB * NP) dt_kernel(CfdMesh m, const double
     commit_keys(red, acc + 2);
     return;
   }
-  // several instances, one group of elements per block: they start at multiples
-  // of 64, or the block's elements commit one by one
-  const int e0 = blockIdx.x * DT_EPB, e = e0 + lane;
-  const int inst = e < m.num_elements ? m.instance[e] : -1, first = m.instance[e0];
-  if (inst >= 0) {
-    node(e);
-    keys();
+  // several instances: each block takes a run of neighbouring groups and commits
+  // where the instance changes (a commit per group: 207 us for the 24 instances
+  // above). They start at multiples of 64, or a group's elements commit one by one.
+  auto clear = [&]() {
+    red.init();
+    rm = pm = dm = INFINITY;
+  };
+  int owner = -1;  // of what has been gathered (uniform in the block)
+  auto flush = [&]() {
+    if (owner >= 0) {
+      keys();
+      commit_keys(red, acc + 3 * owner + 2);
+      __syncthreads();
+    }
+    clear();
+    owner = -1;
+  };
+  const int groups = (m.num_elements + DT_EPB - 1) / DT_EPB, run = (groups + gridDim.x - 1) / gridDim.x;
+  const int last = min(groups, ((int)blockIdx.x + 1) * run);
+  for (int g = blockIdx.x * run; g < last; ++g) {
+    const int e = g * DT_EPB + lane, first = m.instance[g * DT_EPB];
+    const int inst = e < m.num_elements ? m.instance[e] : -1;
+    if (__syncthreads_and(inst < 0 || inst == first)) {
+      if (first < 0) continue;
+      if (first != owner) flush();
+      owner = first;
+      if (inst >= 0) node(e);
+    } else {
+      flush();
+      if (inst >= 0) {
+        node(e);
+        keys();
+        commit_one(red, acc + 3 * inst + 2);
+      }
+      clear();
+    }
   }
-  if (__syncthreads_and(inst < 0 || inst == first)) {
-    if (first >= 0) commit_keys(red, acc + 3 * first + 2);
-  } else if (inst >= 0) {
-    commit_one(red, acc + 3 * inst + 2);
-  }
+  flush();
 }
 
-// The same in FP32-mixed: one thread per element. The wave speed is a handful of
-// single-precision operations there and the pass is bound by its loads, which a
-// thread's 60 independent ones keep in flight: 110 us at 1.05 M elements (252 MB)
-// where one thread per node took 153, 13.0 us at 2,000 where it took 13.4.
+// The same with one thread per element, in FP32-mixed.
 constexpr int DT_BS = 128;
 __global__ void __launch_bounds__(DT_BS) dt_element_kernel(CfdMesh m, const float* __restrict__ q, CfdStageAcc* acc,
                                                            double gamma) {
@@ -428,15 +464,16 @@ static void launch_limit(const CfdSolver* s, LimitParams p, cudaStream_t st) {
   if (s->precision == CFD_FP64) launch_limit_lim<double>(p, s->limiter, st);
   else launch_limit_lim<float>(p, s->limiter, st);
 }
+template <typename R>
+static void launch_dt_nodes(const CfdSolver* s, const void* q, cudaStream_t st) {
+  const unsigned g = blocks_for(s->mesh.num_elements, DT_EPB);
+  dt_kernel<R><<<g > DT_BLOCKS ? DT_BLOCKS : g, DT_EPB * NP, 0, st>>>(s->mesh, (const R*)q, s->acc, s->gamma);
+}
 static void launch_dt(const CfdSolver* s, const void* q, cudaStream_t st) {
   const int n = s->mesh.num_elements;
-  if (s->precision == CFD_FP64) {
-    const unsigned g = blocks_for(n, DT_EPB);
-    dt_kernel<<<!s->mesh.instance && g > DT_BLOCKS ? DT_BLOCKS : g, DT_EPB * NP, 0, st>>>(s->mesh, (const double*)q, s->acc,
-                                                                                         s->gamma);
-  } else {
-    dt_element_kernel<<<blocks_for(n, DT_BS), DT_BS, 0, st>>>(s->mesh, (const float*)q, s->acc, s->gamma);
-  }
+  if (s->precision == CFD_FP64) launch_dt_nodes<double>(s, q, st);
+  else if (n <= (s->mesh.instance ? DT_NODE_MAX32_BATCH : DT_NODE_MAX32)) launch_dt_nodes<float>(s, q, st);
+  else dt_element_kernel<<<blocks_for(n, DT_BS), DT_BS, 0, st>>>(s->mesh, (const float*)q, s->acc, s->gamma);
 }
 static void reset_acc(const CfdSolver* s, cudaStream_t st) {
   const int n = 3 * s->mesh.num_instances;

@@ -1,6 +1,7 @@
 """cfd_time_step and the initial-state check on finite, non-finite and inadmissible states, at the sizes
-where the FP64 pass (one thread per node) takes one element group a block and where its blocks sweep
-(from 18,944 elements), and with several instances aligned to blocks and not."""
+where the pass by node takes one element group a block and where its blocks sweep (from 9,472 elements),
+where FP32-mixed turns to a thread per element (300,000, and 20,000 with several instances), and with
+instances aligned to blocks and not."""
 
 from __future__ import annotations
 
@@ -12,7 +13,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 GAMMA = 1.4
-MESHES = [(1, 1), (7, 5), (96, 98), (97, 98), (400, 250)]  # 2, 70, 18,816, 19,012 and 200,000 elements
+# 2, 70, 9,472 and 9,498, 200,000, 300,000 and 300,600 elements
+MESHES = [(1, 1), (7, 5), (74, 64), (1583, 3), (400, 250), (500, 300), (501, 300)]
 # node, variable and value put into one element
 POISON = {"nan density": (6, 0, np.nan), "nan momentum": (0, 1, np.nan), "nan energy": (14, 3, np.nan),
           "infinite energy": (3, 3, np.inf), "minus infinite energy": (3, 3, -np.inf), "infinite density": (9, 0, np.inf),
@@ -74,17 +76,19 @@ def test_time_step_of_any_state(nx, ny, precision):
 
 
 @pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("nx,ny,starts", [(23, 13, (192, 448)), (150, 100, (64, 19968)), (150, 100, (9984, 29952))])
 @pytest.mark.parametrize("precision", ["fp64", "fp32_mixed"])
-def test_time_step_of_each_instance(precision, aligned):
+def test_time_step_of_each_instance(precision, aligned, nx, ny, starts):
     """Three instances in one launch, their elements starting at multiples of 64 (a block's elements
-    belong to one) or anywhere: each instance's step is its own, and a NaN poisons only its own."""
+    belong to one) or anywhere: each instance's step is its own, and a NaN poisons only its own. With
+    30,000 elements a block of the FP64 pass takes several groups and meets the next instance among them."""
     import torch
 
     from cfd_demo_b200 import _native
 
-    s = _solver(23, 13, precision)  # 598 elements
+    s = _solver(nx, ny, precision)
     q = _state(s)
-    first = np.array([0, 192, 448]) if aligned else np.array([0, 201, 403])
+    first = np.array([0, *starts]) + (np.array([0, 9, 11]) if not aligned else 0)
     owner = np.searchsorted(first, np.arange(q.shape[1]), side="right") - 1
     table = torch.full((s.operators.ld,), -1, dtype=torch.int32, device="cuda")
     table[: q.shape[1]] = torch.from_numpy(owner.astype(np.int32)).cuda()
@@ -96,7 +100,7 @@ def test_time_step_of_each_instance(precision, aligned):
     for poisoned in (None, 0, 1, 2):
         bad = q.copy()
         if poisoned is not None:
-            bad[4, first[poisoned] + 70, 3] = np.nan
+            bad[4, first[poisoned] + 30, 3] = np.nan
         dt = torch.zeros(3, dtype=torch.float64, device="cuda")
         check = torch.zeros(9, dtype=torch.float64, device="cuda")
         x, stream = s.upload(bad), torch.cuda.current_stream().cuda_stream
