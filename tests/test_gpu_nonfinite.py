@@ -40,3 +40,25 @@ def test_finite_entries_of_the_right_hand_side_are_the_oracles(nx, ny, flux):
     got, _ = s.rhs(q)
     assert not np.isfinite(want).all()
     assert np.array_equal(np.isfinite(got), np.isfinite(want))
+
+
+# 70, 9,150, 19,200, 72,900 and 100,352 elements: every form of the stage kernel and of the limiter
+@pytest.mark.parametrize("nx,ny,limiter", [(7, 5, "minmod"), (7, 5, "unlimited"), (75, 61, "minmod"), (75, 61, "unlimited"),
+                                           (96, 100, "unlimited"), (270, 135, "minmod"), (224, 224, "unlimited")])
+@pytest.mark.parametrize("precision", ["fp64", "fp32_mixed"])
+def test_steps_of_bad_states_are_those_of_the_pair_kernel(nx, ny, limiter, precision):
+    """A step from a state with a NaN, an infinity or an inadmissible node: the same verdict, the same
+    NaN minima and the same finite entries as with the register-only pair kernel."""
+    from tests.test_gpu_stage_forms import _solver, _state
+
+    a, b = (_solver(nx, ny, "hllc", limiter, precision, v) for v in (0, 2))
+    q = _state(a, False)
+    k = q.shape[1]
+    for node, var, value in POISON + [(0, 3, np.nan), (2, 1, np.nan), (12, 0, -0.5), (6, 3, 1e-3)]:
+        bad = q.copy()
+        bad[node, [0, k // 3 + 1, k - 1], var] = value
+        (qa, ra), (qb, rb) = a.step(bad, 1e-4), b.step(bad, 1e-4)
+        assert ra.admissible == rb.admissible
+        assert np.isnan(ra.min_density) == np.isnan(rb.min_density)
+        assert np.isnan(ra.min_pressure) == np.isnan(rb.min_pressure)
+        assert np.array_equal(np.isfinite(qa), np.isfinite(qb))
