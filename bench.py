@@ -57,17 +57,17 @@ FALLBACK_HBM_GBS = 6650.0
 # neighbour's own read).
 # DRAM bytes per element of each stage launch (dram__bytes_read.sum +
 # dram__bytes_write.sum) measured by ncu on the autotuned stage kernels (FP32
-# shape 9, FP64 shape 5) at 512x512 quads (K = 524,288; the 724x724 workload
-# is too large for a full capture),
+# shape 9, FP64 shape 0: four lanes per element) at 512x512 quads (K = 524,288;
+# the 724x724 workload is too large for a full capture),
 # scaled to a launch of the benchmark by its element count (traffic grows in
 # proportion to K). Writes still in L2 when a launch ends are not counted
 # there, so the stage result's 240 / 480 B appear partly.
-NCU_BYTES_PER_ELEMENT = {"fp32_mixed": (480.2, 739.5, 750.5), "fp64": (1007.3, 1522.3, 1528.0)}
+NCU_BYTES_PER_ELEMENT = {"fp32_mixed": (480.2, 739.5, 750.5), "fp64": (1018.7, 1516.6, 1526.7)}
 # Warp instructions issued per element of each stage launch (ncu
 # smsp__inst_executed.sum / K, same captures). With 148 SMs issuing at most
 # 4 warp instructions per cycle each, they bound a launch from below at
 # instructions / (148 * 4 * SM clock): the instruction-issue roofline.
-NCU_WARP_INSTRUCTIONS_PER_ELEMENT = {"fp32_mixed": (267.0, 289.2, 304.9), "fp64": (512.1, 527.1, 581.3)}
+NCU_WARP_INSTRUCTIONS_PER_ELEMENT = {"fp32_mixed": (267.0, 289.2, 304.9), "fp64": (448.9, 473.9, 536.5)}
 SMS, ISSUE_PER_SM_CYCLE = 148, 4
 
 

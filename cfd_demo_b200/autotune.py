@@ -2,7 +2,8 @@
 
 The fused stage kernel comes in these shapes (CfdSolver.variant):
   0  chosen by the library from the mesh's size: one thread per node on small
-     meshes, the tile shape that is usually fastest on larger ones
+     meshes; above, four lanes per element or tiles of 32 in FP64, tiles of 32
+     (shape 9 for large unlimited steps) in FP32-mixed
   1  tiled, 32 elements (64 threads) per block, state, geometry and stage base
      staged in shared memory
   2  register-only pair kernel (block size 64/128/256 threads)

@@ -408,27 +408,31 @@ constexpr int LIMIT_BS = 128;
 //   tube,    32,000, FP32              170           -         97         93      93
 //   channel, 10,000, FP64               -            -        138        173     218
 //   channel, 40,000, FP64              279           -        231        262     321
-//   tube,   800,000, FP64            3,373           -         -          -     3,236
+//   tube,    72,000, FP64               -            -        308        295     289
+//   channel, 90,000, FP64               -            -        337        372     439
+//   waves,  500,000, FP64               -            -      1,578      1,524   1,564
+//   tube,   800,000, FP64               -            -      2,458      2,335   2,280
 // (two launches here: a scan of the whole mesh, then a rewrite of a global list with
 // four lanes an element.)
 // A block that rewrites all it scans takes EPB / 8 rounds of some 4,900 cycles,
 // so few elements a block balance better while the blocks fit the GPU at once
-// (seven of them an SM at 72 registers); in an attempt the direct form is never slower
-// while its blocks of eight elements are one wave (8,288), and on large meshes the
-// fixed work of a block counts instead. There a troubled region is then a long
-// chain in a few blocks, which in FP32-mixed, with its faster stages, made the
-// attempt slower than a rewrite of a global list. FP32-mixed meshes above LIMIT_SCAN32_MAX therefore scan
-// and rewrite in two launches, the listed elements dealt out one by one to the half
-// warps of the grid. One attempt, us (FP32-mixed; channel and waves: many troubled
-// elements side by side, tube: few):
+// (seven of them an SM at 72 registers); in an attempt the direct form is never
+// slower while its blocks of eight elements are one wave (8,288), and on large
+// meshes the fixed work of a block counts instead. There a troubled region is a
+// long chain in a few blocks, which in FP32-mixed, with its faster stages, made the
+// attempt slower than a rewrite of a global list. FP32-mixed meshes above
+// LIMIT_SCAN32_MAX therefore scan and rewrite in two launches, the listed elements
+// dealt out one by one to the half warps of the grid. One attempt, us (FP32-mixed;
+// channel and waves: many troubled elements side by side, tube: few):
 //                       four lanes, global list   scan of 32   of 64   of 128   two launches
 //   tube,     72,000               219                172        161      155        165
 //   channel,  90,000               231                204        226      272        183
 //   waves,   180,000               482                431        438      470        371
 //   waves,   500,000               942                989        939      976        831
 //   tube,    800,000             1,384              1,463      1,325    1,258      1,259
-// In FP64 the single launch was nowhere slower than the four-lane rewrite (channel,
-// 90,000: 439 against 530) and stays.
+// In FP64 the single launch was nowhere slower than the four-lane rewrite (a limiter
+// call on the channels of 72,000 and 90,000 elements: 63 and 82 us against 60 and
+// 71) and stays; its line between scans of 32 and of 128 is a compromise.
 constexpr int LIMIT_DIRECT_MAX = 148 * 7 * (LIMIT_BS / HALF), LIMIT_SCAN32_MAX = 70000;
 constexpr int LIMIT_REWRITE_BLOCKS = 148 * 3;  // 3,552 half warps; seven blocks an SM cost a tube 2 % more
 template <typename R, int PHI, int EPB>

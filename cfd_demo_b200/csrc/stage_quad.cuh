@@ -23,12 +23,13 @@
 // handed out as it is: there a sum of zero times every flux carries a non-finite
 // one to all rows of its element, as the dense products of the reference do.
 //
-// What bounds it: instruction issue and the latency of double-precision chains
-// (the FP64 pipe is 41 % busy, 51 % of the issue slots, 16 warps an SM). Two
-// lanes per element, each forming every node's primitives and flux, issue 512
-// warp instructions an element and stage; this form 474 (562 before the tables
-// were laid out for 16-byte constant loads and the density reciprocals were
-// kept from the volume term). One thread per element issues 346 but has 8 warps
+// What bounds it: instruction issue and the latency of double-precision chains and
+// of shared memory (Roe, unlimited, 524,288 elements: the FP64 pipe is 43-45 % busy,
+// 52-54 % of the issue slots, 16 warps an SM). Two lanes per element, each forming
+// every node's primitives and flux, issue 512 / 527 / 581 warp instructions an
+// element (stages 1 / 2 / 3); this form 449 / 474 / 537 (562 in the second before
+// the tables were laid out for 16-byte constant loads and the density reciprocals
+// were kept from the volume term). One thread per element issues 346 but has 8 warps
 // an SM and ran no faster than the tiles. One RK3 attempt (graph replay), us:
 //   elements                              tiles of 32   of 64   this form
 //   32,000    hllc/van_leer                   213         237       167

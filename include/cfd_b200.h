@@ -218,7 +218,8 @@ typedef struct CfdSolver {
     CfdControl* control;   /* [num_instances] */
     int32_t block_size;    /* threads per block of the pair stage kernel (64, 128, 256); 0 = default */
     int32_t variant;       /* stage kernel: 0 chosen by the size of the mesh (default: one thread per
-                              node on small meshes, else a tiled shape), 1 tiled (32 elements per
+                              node on small meshes; above, four lanes per element or tiles of 32
+                              in FP64, tiles of 32 or 64 in FP32-mixed), 1 tiled (32 elements per
                               block) + staged base rows,
                               2 register-only pair kernel, 3 tiled with 64 elements per block,
                               4 tiled with registers capped for more resident blocks,
@@ -319,8 +320,8 @@ int cfd_rk3_advance(const CfdSolver* s, void* x0, void* x1, void* stage, int32_t
  * tiles of all instances, with a grid-wide barrier between the phases of an
  * attempt (zero the reduction slots; stage k and its limiter passes for
  * k = 1, 2, 3; report and control). Returns early once no instance is active.
- * Needs the limit_list scratch. The
- * tile shape is fixed per precision (FP32: variant 9, FP64: variant 3) and the
+ * Asks for the limit_list scratch, and for buffers that whole tiles fit (see
+ * CfdMesh.ld). The tile shape is fixed per precision (FP32: variant 9, FP64: variant 3) and the
  * per-element arithmetic is that of the separate launches, so the results
  * equal those of `attempts` x (cfd_rk3_attempt + cfd_run_control) with that
  * variant: bit for bit in FP32-mixed, to the last bits in FP64 (where the
